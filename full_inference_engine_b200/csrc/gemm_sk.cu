@@ -1,40 +1,46 @@
 // Persistent stream-K weight-only linear for decode-sized token counts (M <= 64) on sm_100a.
 //
-// The problem is cut into UNITS of one weight tile x one K block (128 output channels x 128
-// K: 8 KB of packed int4, 16 KB of int8).  The grid is at most one block per SM and block b
+// The problem is cut into UNITS of 16 KB: one weight tile of 128 output channels x 256 K of packed
+// int4 (two K blocks) or 128 K of int8 (one).  The grid is one or two blocks per SM and block b
 // owns the contiguous unit range [b U / G, (b + 1) U / G) in (tile, K block) order, so every
 // block streams the same number of weight bytes whatever the shape: there is no tail wave and
 // no split-K plan.  A run of a block's units inside one tile is a SEGMENT; a segment that
 // covers the tile's whole K is stored directly.  Otherwise the first block of the tile (the
 // one whose range ENDS in it, so it gets there last) owns the output: it adds the partials of
-// the tile's other blocks to its own accumulator in block order — fixed order, so results are
-// reproducible — and stores.  The others park their fp32 partials in the workspace as
+// the tile's other blocks to its own accumulator in a fixed order, so that results are
+// reproducible, and stores.  The others park their fp32 partials in the workspace as
 // self-validating words (a word of 0 means "not written"), which the owner polls directly:
 // no fence, no flag, no atomic, because under a saturated memory system every dependent trip
 // to L2 costs about a microsecond.  An owner only ever waits for higher-numbered blocks of its
-// own grid (bounded), and the grid is at most one block per SM, so they are resident.
+// own grid (bounded), and the grid is at most what fits the GPU at once (a block takes at most
+// half an SM where there are two per SM), so they are resident.
 //
-// A block uses at most half of an SM (448 threads, <= 72 registers, <= 113 KB of shared
-// memory when the ring allows it, 256 TMEM columns), so the NEXT kernel of the stream
+// Bound: HBM (the weights), so the work per weight byte must stay under the issue, shared-memory
+// and mma.sync budgets of an SM: a unit arrives every ~700 cycles at 6.5 TB/s.  The multiply
+// is a warp-level mma.sync with the weights as its A operand: a consumer warp reads its packed
+// rows from shared memory, unpacks them in registers straight into A fragments and multiplies,
+// with no hand-over to another warp.  (The tcgen05 form of this kernel had to write the unpacked
+// operand to tensor memory and pass it to an MMA thread, ~1300 cycles for the same bytes.)
+//
+// 4-bit weights enter the multiply as the format's fp16 product (fp16 activations) or as the exact integers
+// n - zero with the group's scale applied to the group's fp32 sum (bf16 activations); int8 weights enter as
+// they are and the channel scale is applied at the end.
+//
+// A block uses at most half of an SM up to 16 token rows, so the NEXT kernel of the stream
 // (programmatic dependent launch) becomes resident beside it and pre-fills its own weight
 // ring while this one drains: the HBM stream does not stop at kernel boundaries.
 //
 // Warp roles:
-//   warp 0       TMA producer feeding three rings: per unit one box of packed weights
-//                (64-byte swizzle); per eight K blocks of a tile one box of scales (and
-//                zero-points) [128 rows x 8 groups]; per unit one box of activations ([2 atoms]
-//                x [TOK rows] x [64 elements], 128-byte swizzle).  With static weights the
-//                weight and scale rings fill BEFORE the stream-order wait, and the dequantise
-//                groups already unpack them into tensor memory; only the activations wait
-//   warp 1       TMEM allocation, tcgen05.mma issue (one elected thread), commits
-//   warps 2-5    epilogue: tcgen05.ld of a finished segment (the accumulator is handed back
-//                to the MMA warp as soon as it is in registers), then park the partial, or
-//                collect the other blocks' partials, scale/bias and store
-//   warps 6-13   two dequantise groups of four warps; a group takes every other unit, each
-//                thread one output channel (its TMEM lane) x the unit's 128 K: packed row out
-//                of shared memory, unpack in registers, A operand (activation dtype) into tensor memory
-//
-// D[128 channels, TOK] (fp32, TMEM) += Wd[128, 16] (TMEM) * X[TOK, 16]^T (smem).
+//   warp 0       TMA producer of the weights: per unit one box of packed weights (64-byte
+//                swizzle), per eight K blocks of a tile one box of scales (and zero-points)
+//                [128 rows x 8 groups].  With static weights both rings fill BEFORE the
+//                stream-order wait
+//   warp 1       TMA producer of the activations: per unit one box of [2 or 4 atoms] x [TOK rows]
+//                x [64 elements], 128-byte swizzle, behind the stream-order wait
+//   the others   consumer groups; a group takes every G-th unit, a warp 16 MT channels of it x
+//                the unit's 128 K x all token rows.  At the end of a segment the groups hand
+//                their sums to group 0 through shared memory, and group 0 parks the partial,
+//                or adds the other blocks' and stores
 //
 // Reference counterparts: _w4a16_gemv_kernel / _w4a16_linear_kernel
 // (engine/kernels/w4a16_linear.py:27-74, 120-177) and _w8a16_linear_kernel
@@ -42,26 +48,32 @@
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "tc_common.cuh"
 
 namespace b200q {
 
-constexpr int kSkGroups = 2;                                   // dequantise groups
-constexpr int kSkThreads = 32 * (2 + 4 + 4 * kSkGroups);       // 448
-constexpr int kSkMaxStages = 16;                               // weight ring
-constexpr int kSkXStages = 4;                                  // activation ring (most; wide token tiles take two)
+constexpr int kSkProducers = 2;                                // weights (and scales), activations
+constexpr int kSkTiles = 2;                                    // 16-channel MMA tiles per consumer warp
+constexpr int kSkGroups = 2;                                   // consumer groups
+constexpr int kSkMaxStages = 12;                               // ring of units: weights and activations
 constexpr int kSkSStages = 3;                                  // scale-chunk ring (4-bit formats)
-constexpr int kSkAStages = 3;                                  // operand stages in tensor memory
+// K blocks of 128 per unit.  4-bit weights take two where the registers allow it: the waits and the
+// bookkeeping of a unit cost a third of its instructions with one (24576 x 4096, one row: 17.4 us
+// with one, 15.1 us with two unrolled; 16 rows: 21.0 and 21.3 us, but 8.8 and 9.9 us on 6144 x 4096).
+__host__ __device__ constexpr int sk_sub(int format, int nt) { return format == FMT_W8 || nt == 2 ? 1 : 2; }
+// 64-byte K chunks of a weight row per unit: the depth of its TMA box
+__host__ __device__ constexpr int sk_depth(int format, int nt) { return format == FMT_W8 ? 2 : sk_sub(format, nt); }
 constexpr int kSkMaxTok = 64;
-constexpr int kSkTmemCols = 256;                               // accumulator [0, 64), operand stages [64, 256)
-constexpr int kSkACol0 = 64;
-constexpr int kSkBarrierBytes = 512;
-static_assert(8 * (2 * kSkMaxStages + 2 * kSkXStages + 2 * kSkSStages + 2 * kSkAStages + 3) + 16 <= kSkBarrierBytes,
-              "the barrier region holds every ring's barriers");
-static_assert(kSkACol0 + 64 * kSkAStages <= kSkTmemCols, "operand stages fit the tensor memory allocation");
-constexpr int kSkMaxGrid = 160;                                // blocks the exchange region has slots for
-static_assert(static_cast<size_t>(kSkMaxGrid) * kSkMaxTok * kBlockN * sizeof(uint32_t) <= kWsExchangeBytes,
+constexpr int kSkBarrierBytes = 1024;                          // (keeps the weight ring 1024-byte aligned)
+constexpr int kSkMaxArgmaxRows = 32;
+constexpr int kSkBestOffset = 704;                             // [32] best keys of a block's tiles (argmax only)
+static_assert(8 * (5 * kSkMaxStages + 2 * kSkSStages + 16) + 16 <= kSkBestOffset &&
+                  kSkBestOffset + 8 * kSkMaxArgmaxRows <= kSkBarrierBytes,
+              "the barrier region holds every ring's barriers and the argmax keys");
+constexpr int kSkMaxSms = 160;                                 // one block each, or two of up to 16 token rows
+static_assert(static_cast<size_t>(kSkMaxSms) * kSkMaxTok * kBlockN * sizeof(uint32_t) <= kWsExchangeBytes,
               "the exchange region holds one partial per block");
 constexpr size_t kSkHalfSm = 115712;                           // (228 KiB - 2 x 1 KiB reserved) / 2
 constexpr size_t kSkFullSm = 226 * 1024;
@@ -74,14 +86,15 @@ struct SkParams {
   void* y;
   int64_t ldy;
   int M, N, K;
-  int tok;               // UMMA N: token rows per tile, multiple of 16, <= 64
-  int kb_total;          // K / 128
-  uint32_t total_units;  // weight tiles x K blocks
-  int stages;            // weight ring depth
-  int x_stages;          // activation ring depth
-  uint32_t idesc;
+  int kb_total;          // units along K
+  uint32_t total_units;  // weight tiles x units along K
+  int stages;            // ring depth
   int static_weights;
   int swiglu;
+  int vec_out;           // a lane's neighbouring outputs of a row may be stored at once
+  int argmax;            // y is int64 channel[M]: per row the channel of the largest output (M <= 32)
+  unsigned long long* row_keys;  // [M] in the workspace, zero between launches (argmax only)
+  unsigned* counter;     // zero between launches (argmax only)
   uint32_t* exchange;    // [grid][tok][128] encoded fp32 partials, all zero between launches
   unsigned* status;
 };
@@ -101,108 +114,317 @@ __device__ __forceinline__ uint32_t sk_first_unit(uint32_t block, uint32_t grid,
 __device__ __forceinline__ uint32_t sk_encode(float v) { return __float_as_uint(v + 0.0f) ^ 0x80000000u; }
 __device__ __forceinline__ float sk_decode(uint32_t w) { return __uint_as_float(w ^ 0x80000000u); }
 constexpr uint32_t kSkExchangePolls = 1u << 15;          // x ~1 us per look: gives up after tens of milliseconds
-__device__ __forceinline__ uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Untiled bulk copy global -> shared of this block (both 16-byte aligned, size a multiple of
-// 16 bytes), completion on an mbarrier.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+// The two or four neighbouring channels of one lane, as one access.
+__device__ __forceinline__ void ld_exchange(uint32_t (&v)[4], const uint32_t* p) {
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "l"(p)
                : "memory");
 }
-// AND of a predicate over the 128 epilogue threads (named barrier 1).
-__device__ __forceinline__ bool epilogue_all(bool mine) {
-  uint32_t out;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 q, %1, 0;\n"
-      "bar.red.and.pred p, 1, 128, q;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(out)
-      : "r"(static_cast<uint32_t>(mine))
-      : "memory");
-  return out != 0;
+__device__ __forceinline__ void ld_exchange(uint32_t (&v)[2], const uint32_t* p) {
+  asm volatile("ld.relaxed.gpu.global.v2.u32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p) : "memory");
 }
-__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+__device__ __forceinline__ void st_exchange(uint32_t* p, const uint32_t (&v)[4]) {
+  __stcg(reinterpret_cast<uint4*>(p), make_uint4(v[0], v[1], v[2], v[3]));
+}
+__device__ __forceinline__ void st_exchange(uint32_t* p, const uint32_t (&v)[2]) {
+  __stcg(reinterpret_cast<uint2*>(p), make_uint2(v[0], v[1]));
+}
+__device__ __forceinline__ void st_shared_f(uint32_t addr, const float (&v)[4]) {
+  asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+}
+__device__ __forceinline__ void st_shared_f(uint32_t addr, const float (&v)[2]) {
+  asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(addr), "f"(v[0]), "f"(v[1]) : "memory");
+}
+__device__ __forceinline__ void ld_shared_f(float (&v)[4], uint32_t addr) {
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ld_shared_f(float (&v)[2], uint32_t addr) {
+  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ void st_shared_f32(uint32_t addr, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+
+__device__ __forceinline__ unsigned short half_bits(uint32_t two, int which) {
+  return static_cast<unsigned short>(which ? two >> 16 : two & 0xFFFFu);
 }
 
-template <int FMT, typename T>
-__global__ void __launch_bounds__(kSkThreads, 2)
-wq_gemm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
-                  const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_z,
-                  const SkParams p) {
+// The fused argmax of one token over a warp's channels: the values as the plain call would store them -> an
+// order-preserving 16-bit code; key = code << 32 | (0xFFFFFFFF - channel), so the largest value wins and
+// ties go to the smallest channel; the best of the eight lanes that hold the token (t, t + 4, ...) into *best.
+// Not inlined: the plain calls' registers do not pay for it.
+template <typename T, int N>
+struct LaneValues {
+  float v[N];
+};
+template <typename T, int N>
+__device__ __noinline__ void argmax_token(LaneValues<T, N> values, int n, int limit, bool wanted, uint32_t best) {
+  unsigned long long key = 0ull;
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    const uint32_t two = pack_pair<T>(values.v[e], values.v[e]);
+    const uint32_t code = (two & 0x8000u) ? (~two & 0xFFFFu) : ((two & 0xFFFFu) | 0x8000u);
+    const unsigned long long mine = (static_cast<unsigned long long>(code) << 32) | (0xFFFFFFFFull - static_cast<uint32_t>(n + e));
+    if (n + e < limit && mine > key) key = mine;
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
+    if (other > key) key = other;
+  }
+  if (wanted && key != 0ull && (threadIdx.x & 31) < 4)
+    asm volatile("red.shared.max.u64 [%0], %1;" ::"r"(best), "l"(key) : "memory");
+}
+
+// D[16 channels, 8 tokens] = A[16 channels, 16 K] * B[16 K, 8 tokens] + C, fp32 accumulation.
+template <typename T>
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0,
+                                          float c1, float c2, float c3);
+template <>
+__device__ __forceinline__ void mma_16816<__half>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1,
+                                                  float c0, float c1, float c2, float c3) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+template <>
+__device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                                         uint32_t b1, float c0, float c1, float c2, float c3) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// ---------------------------------------------------------------- exact integers as MMA operands
+// Nibbles n at bits 0-3 or 4-7 of both halves of a word -> a pair of MMA operands.
+//
+// fp16: 0x6400 | n = 1024 + n for the low nibble, 1024 + 16 n for the high one (times 1/16, minus
+// 64 + zero), then ONE multiply by the group's fp16 scale: the format's own product
+// (unpack_w4_reference, engine/kernels/w4a16_format.py:53-69), bit for bit.
+//
+// bf16: the exact integer (n - zero) / kInverseUnit.  The format's product would have to be rounded once
+// more, to bf16; instead the tensor core sums a group's products with the integers in fp32 and the
+// scale is applied to that sum (relative error against 64 bits of a 4096-deep projection: 1.7e-3, of which
+// the output's rounding is nearly all, against 2.4e-3).  bf16 has seven mantissa bits, too few for the
+// encoding above: the masked bits are taken as the subnormals n 2^-133 and 16 n 2^-133 and one FMA lifts them
+// to n 2^-6, minus zero 2^-6.
+template <typename T>
+struct Nibbles;
+template <>
+struct Nibbles<__half> {
+  static constexpr bool kScaled = true;
+  static constexpr float kInverseUnit = 1.0f;
+  uint32_t lo_c, hi_c, scale;
+  __device__ __forceinline__ Nibbles(float zero, unsigned short s)
+      : lo_c(as_u32(__float2half2_rn(1024.0f + zero))), hi_c(as_u32(__float2half2_rn(-(64.0f + zero)))),
+        scale(s | (static_cast<uint32_t>(s) << 16)) {}
+  __device__ __forceinline__ uint32_t lo(uint32_t u) const {
+    return as_u32(__hmul2(__hsub2(as_h2(lop3_and_or(u, 0x000F000Fu, 0x64006400u)), as_h2(lo_c)), as_h2(scale)));
+  }
+  __device__ __forceinline__ uint32_t hi(uint32_t u) const {
+    return as_u32(__hmul2(__hfma2(as_h2(lop3_and_or(u, 0x00F000F0u, 0x64006400u)), __float2half2_rn(0.0625f), as_h2(hi_c)),
+                          as_h2(scale)));
+  }
+};
+__device__ __forceinline__ __nv_bfloat162 as_bf2(uint32_t u) { return *reinterpret_cast<__nv_bfloat162*>(&u); }
+template <>
+struct Nibbles<__nv_bfloat16> {
+  static constexpr bool kScaled = false;
+  static constexpr float kInverseUnit = 64.0f;
+  uint32_t c;
+  __device__ __forceinline__ Nibbles(float zero, unsigned short) : c(as_u32(__float2bfloat162_rn(zero * -0.015625f))) {}
+  __device__ __forceinline__ uint32_t lo(uint32_t u) const {
+    return as_u32(__hfma2(as_bf2(u & 0x000F000Fu), as_bf2(0x7F007F00u), as_bf2(c)));    // x 2^127
+  }
+  __device__ __forceinline__ uint32_t hi(uint32_t u) const {
+    return as_u32(__hfma2(as_bf2(u & 0x00F000F0u), as_bf2(0x7D007D00u), as_bf2(c)));    // x 2^123
+  }
+};
+__device__ __forceinline__ uint32_t bf16_sub2(uint32_t a, uint32_t b) { return as_u32(__hsub2(as_bf2(a), as_bf2(b))); }
+// Four int8 -> two pairs in K order.  fp16: int8x4_to_h2.  bf16: (128 + (q & 127)) - (128 or 256),
+// the subtrahend picked by the sign bit (0x4300 is 128, 0x4380 is 256): both terms and the
+// difference are exact.
+template <typename T>
+__device__ __forceinline__ void int8_pairs(uint32_t w, uint32_t& k01, uint32_t& k23);
+template <>
+__device__ __forceinline__ void int8_pairs<__half>(uint32_t w, uint32_t& k01, uint32_t& k23) {
+  __half2 a, b;
+  int8x4_to_h2(w, a, b);
+  k01 = as_u32(a);
+  k23 = as_u32(b);
+}
+template <>
+__device__ __forceinline__ void int8_pairs<__nv_bfloat16>(uint32_t w, uint32_t& k01, uint32_t& k23) {
+  const uint32_t u = prmt(w, 0u, 0x3120);       // bytes (b0,b2,b1,b3): (b0,b1) sit at bits 0 and 16
+  k01 = bf16_sub2(lop3_and_or(u, 0x007F007Fu, 0x43004300u), lop3_and_or(u, 0x00800080u, 0x43004300u));
+  k23 = bf16_sub2(lop3_and_or(u >> 8, 0x007F007Fu, 0x43004300u), lop3_and_or(u >> 8, 0x00800080u, 0x43004300u));
+}
+
+__device__ __forceinline__ uint32_t word_of(const uint4& v, int i) {
+  return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
+}
+
+// The 128 K of a K block are four PIECES of 32: a piece is one 16-byte load of activations per token row and
+// lane (eight consecutive K) and two m16n8k16 steps, lane t of a quad supplying four K of each.
+// Which K a lane supplies is free as long as both operands agree, so it follows the packed row:
+//   REF   lane t holds bytes 16 t .. 16 t + 15: K 16 t + .. (low nibbles) and 64 + 16 t + ..
+//         (high); piece p: bytes 8 (p >> 1) .., low (p even) or high nibbles
+//   W8    piece p: sub-tile p >> 1 (K 0..63, 64..127), bytes 16 t + 8 (p & 1) ..
+//   ASYM  lane t holds words 4 t .. 4 t + 3 = K 32 t .. 32 t + 31; piece p: one word.  Lanes
+//         t >= 2 take their words in the order 2, 3, 0, 1 (the caller swapped them): their
+//         activations come from the other 64-element atom, on the same banks otherwise
+// One row's A registers of piece P: pairs (k01, k23) of the first step, then of the second.
+template <int FMT, typename T, int P>
+__device__ __forceinline__ void unpack_piece(const uint4& row, const Nibbles<T>& z, uint32_t (&out)[4]) {
+  if (FMT == FMT_W4_REF) {
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      // bytes (b0,b1,b2,b3) -> (b0,b2,b1,b3): the masks then pick (b0,b1) from the word and
+      // (b2,b3) from the word shifted by 8
+      const uint32_t u = prmt(word_of(row, 2 * (P >> 1) + w), 0u, 0x3120);
+      out[2 * w] = (P & 1) ? z.hi(u) : z.lo(u);
+      out[2 * w + 1] = (P & 1) ? z.hi(u >> 8) : z.lo(u >> 8);
+    }
+  } else if (FMT == FMT_W4_ASYM) {
+    const uint32_t u = word_of(row, P);
+    out[0] = z.lo(u);
+    out[1] = z.hi(u);
+    out[2] = z.lo(u >> 8);
+    out[3] = z.hi(u >> 8);
+  } else {
+    int8_pairs<T>(word_of(row, 2 * (P & 1)), out[0], out[1]);
+    int8_pairs<T>(word_of(row, 2 * (P & 1) + 1), out[2], out[3]);
+  }
+}
+// Where a lane's activations of piece p lie: XORed into its 16-byte chunk offset, and which of the
+// two 64-element atoms (ASYM: a matter of the lane).
+template <int FMT>
+__device__ __forceinline__ constexpr int piece_flip(int p) {
+  return FMT == FMT_W4_REF ? (p >> 1) << 4 : (FMT == FMT_W4_ASYM ? p << 4 : (p & 1) << 4);
+}
+template <int FMT>
+__device__ __forceinline__ constexpr int piece_atom(int p) {
+  return FMT == FMT_W4_REF ? (p & 1) : (FMT == FMT_W4_ASYM ? 0 : p >> 1);
+}
+
+// The nibble constants of a lane's channels.
+template <typename T, int N>
+struct SkGroup;
+template <typename T>
+struct SkGroup<T, 2> {
+  Nibbles<T> v[2];
+  __device__ __forceinline__ SkGroup(const float (&z)[2], const unsigned short (&s)[2])
+      : v{Nibbles<T>(z[0], s[0]), Nibbles<T>(z[1], s[1])} {}
+  __device__ __forceinline__ const Nibbles<T>& operator[](int i) const { return v[i]; }
+};
+template <typename T>
+struct SkGroup<T, 4> {
+  Nibbles<T> v[4];
+  __device__ __forceinline__ SkGroup(const float (&z)[4], const unsigned short (&s)[4])
+      : v{Nibbles<T>(z[0], s[0]), Nibbles<T>(z[1], s[1]), Nibbles<T>(z[2], s[2]), Nibbles<T>(z[3], s[3])} {}
+  __device__ __forceinline__ const Nibbles<T>& operator[](int i) const { return v[i]; }
+};
+
+// The shape of a block: MT tiles of 16 channels per consumer warp (8 / MT warps cover a weight
+// tile), G consumer groups of that many warps taking units in turn.  NT token tiles of eight.
+template <int FMT, typename T, int NT, int MT, int G>
+struct SkShape {
+  static constexpr bool kGroupSums = FMT != FMT_W8 && !Nibbles<T>::kScaled;   // a group's scale is applied to its sum
+  static constexpr int kRowWarps = 8 / MT;
+  static constexpr int kThreads = 32 * (kSkProducers + kRowWarps * G);
+  static constexpr int kBlocksPerSm = NT <= 2 ? 2 : 1;
+  static constexpr int kSlab = NT <= 2 ? 1 : (FMT != FMT_W8 && NT <= 4 ? 4 : 2);   // pieces unpacked before the multiply
+  static constexpr int kChains = NT * MT == 1 ? 2 : 1;    // a lone chain of MMAs would be bound by their latency
+  static constexpr bool kLocal = kSlab > 1;      // unscaled sums live for one token tile of one slab, not for the unit
+  static constexpr int kGroupTiles = kLocal ? 1 : NT;
+
+  template <int P>
+  __device__ __forceinline__ static void unpack(const uint4 (&rows)[2 * MT], const SkGroup<T, 2 * MT>& z,
+                                                uint32_t (&a)[MT][2][4]) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      uint32_t even[4], odd[4];
+      unpack_piece<FMT, T, P>(rows[2 * mt], z[2 * mt], even);          // MMA rows 0..7
+      unpack_piece<FMT, T, P>(rows[2 * mt + 1], z[2 * mt + 1], odd);   // MMA rows 8..15
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        a[mt][s][0] = even[2 * s];
+        a[mt][s][1] = odd[2 * s];
+        a[mt][s][2] = even[2 * s + 1];
+        a[mt][s][3] = odd[2 * s + 1];
+      }
+    }
+  }
+};
+
+template <int FMT, typename T, int NT, int MT, int G>
+__global__ void __launch_bounds__(SkShape<FMT, T, NT, MT, G>::kThreads, SkShape<FMT, T, NT, MT, G>::kBlocksPerSm)
+wq_gemm_sk_kernel_mma(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
+                      const __grid_constant__ CUtensorMap tm_s, const __grid_constant__ CUtensorMap tm_z,
+                      const SkParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  constexpr int kWBytes = PackedStage<FMT>::kBytes;
+  using Shape = SkShape<FMT, T, NT, MT, G>;
+  constexpr int kRowWarps = Shape::kRowWarps, kChan = 2 * MT;      // kChan: channels per lane
+  constexpr int kSub = sk_sub(FMT, NT);                                // K blocks per unit
+  constexpr int kUnroll = NT == 1 ? kSub : 1;
+  constexpr int kChunkUnits = 8 / kSub;                            // units per scale chunk
+  constexpr int kWBytes = kSub * PackedStage<FMT>::kBytes;
   constexpr bool kGroups = FMT != FMT_W8;                          // per-group scales to fetch
   constexpr int kSBytes = kGroups ? kSkChunkBytes * (FMT == FMT_W4_ASYM ? 2 : 1) : 0;
-  const int x_atom_bytes = p.tok * 128;                            // one 64-wide K atom of [tok x 128 B]
-  const int x_bytes = 2 * x_atom_bytes;
+  constexpr int kTok = 8 * NT;
+  constexpr int kXAtom = kTok * 128;                               // one 64-wide K atom of [tok x 128 B]
+  constexpr int kXBytes = kSub * 2 * kXAtom;
   const int S = p.stages;
-  const uint32_t x_ring = smem_base;                               // 1024-byte aligned atoms
-  const uint32_t w_ring = x_ring + p.x_stages * x_bytes;
-  const uint32_t s_ring = w_ring + S * kWBytes;
-  const uint32_t bars = s_ring + kSkSStages * kSBytes;
-  const uint32_t w_full = bars;                                    // [kSkMaxStages]
-  const uint32_t w_empty = w_full + 8 * kSkMaxStages;              // 4 arrivals: the warps of one group
-  const uint32_t x_full = w_empty + 8 * kSkMaxStages;              // [kSkXStages]
-  const uint32_t x_empty = x_full + 8 * kSkXStages;                // MMA commit
-  const uint32_t s_full = x_empty + 8 * kSkXStages;                // [kSkSStages]
-  const uint32_t s_empty = s_full + 8 * kSkSStages;                // 8 arrivals: every dequantise warp
-  const uint32_t a_full = s_empty + 8 * kSkSStages;                // [kSkAStages], 4 arrivals
-  const uint32_t a_empty = a_full + 8 * kSkAStages;                // MMA commit
-  const uint32_t acc_full = a_empty + 8 * kSkAStages;              // MMA commit
-  const uint32_t acc_empty = acc_full + 8;                         // 4 arrivals: the epilogue warps
-  const uint32_t xg_full = acc_empty + 8;                          // staged partials of other blocks landed
-  const uint32_t tmem_slot = xg_full + 8;
-  const uint32_t abort_slot = tmem_slot + 4;
+  // everything but the rings of weights and activations, which come last, is at a fixed offset
+  const uint32_t bars = smem_base;
+  // A group sees only every G-th unit.  Were there one "full" barrier per slot, a group could wait for a slot's
+  // next filling while the one before (another group's) has not landed yet, and take the parity of
+  // the filling before that for its own.  With G per slot a barrier belongs to one group, in order.
+  const uint32_t w_full = bars;                                    // [G * stages]: unit j at j % (G * stages)
+  const uint32_t x_full = w_full + 8 * G * kSkMaxStages;           // [G * stages]
+  const uint32_t u_empty = x_full + 8 * G * kSkMaxStages;              // one arrival per warp of a group
+  const uint32_t s_full = u_empty + 8 * kSkMaxStages;              // [kSkSStages]
+  const uint32_t s_empty = s_full + 8 * kSkSStages;                // one arrival per consumer warp
+  const uint32_t red_full = s_empty + 8 * kSkSStages;              // [8], one per 16 MT channels: G - 1 arrivals
+  const uint32_t red_empty = red_full + 8 * 8;                     // [8]
+  const uint32_t abort_slot = red_empty + 8 * 8;
+  const uint32_t s_ring = bars + kSkBarrierBytes;                  // [kSkSStages]
+  const uint32_t red = s_ring + kSkSStages * kSBytes;              // the other groups' sums, [tok][128] fp32 each
+  const uint32_t w_ring = red + (G - 1) * kTok * 512;              // [stages], 1024-byte aligned
+  const uint32_t x_ring = w_ring + S * kWBytes;                    // [stages], 1024-byte aligned atoms
   uint8_t* generic_base = smem_raw + (smem_base - smem_u32(smem_raw));
-  volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(generic_base + (tmem_slot - smem_base));
   volatile int* abort_p = reinterpret_cast<volatile int*>(generic_base + (abort_slot - smem_base));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t U = p.total_units, G = gridDim.x;
-  const uint32_t u0 = sk_first_unit(blockIdx.x, G, U);
-  const uint32_t u1 = sk_first_unit(blockIdx.x + 1, G, U);
+  const uint32_t U = p.total_units, grid = gridDim.x;
+  const uint32_t u0 = sk_first_unit(blockIdx.x, grid, U);
+  const uint32_t u1 = sk_first_unit(blockIdx.x + 1, grid, U);
   const int n_units = static_cast<int>(u1 - u0);
   const int KB = p.kb_total;
   const int tile0 = static_cast<int>(u0 / static_cast<uint32_t>(KB));
   const int kbi0 = static_cast<int>(u0 - static_cast<uint32_t>(tile0) * KB);
 
   if (warp == 0) {
-    if (lane < kSkMaxStages) {
+    if (lane < G * kSkMaxStages) {
       mbar_init(w_full + 8 * lane, 1);
-      mbar_init(w_empty + 8 * lane, 4);
-    }
-    if (lane < kSkXStages) {
       mbar_init(x_full + 8 * lane, 1);
-      mbar_init(x_empty + 8 * lane, 1);
     }
+    if (lane < kSkMaxStages) mbar_init(u_empty + 8 * lane, kRowWarps);
     if (lane < kSkSStages) {
       mbar_init(s_full + 8 * lane, 1);
-      mbar_init(s_empty + 8 * lane, 4 * kSkGroups);
+      mbar_init(s_empty + 8 * lane, kRowWarps * G);
     }
-    if (lane < kSkAStages) {
-      mbar_init(a_full + 8 * lane, 4);
-      mbar_init(a_empty + 8 * lane, 1);
+    if (lane < 8) {
+      mbar_init(red_full + 8 * lane, G - 1);
+      mbar_init(red_empty + 8 * lane, 1);
     }
+    reinterpret_cast<unsigned long long*>(generic_base + kSkBestOffset)[lane] = 0ull;
     if (lane == 0) {
-      mbar_init(acc_full, 1);
-      mbar_init(acc_empty, 4);
-      mbar_init(xg_full, 1);
       *abort_p = 0;
       tma_prefetch_desc(&tm_w);
       tma_prefetch_desc(&tm_x);
@@ -211,517 +433,475 @@ wq_gemm_sk_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
     mbar_fence_init();
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, kSkTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
   __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot_p;
   // Let the next kernel of the stream become resident now; it orders itself behind this grid
   // with griddepcontrol.wait before it touches anything this grid writes.
   if (threadIdx.x == 0) grid_launch_dependents();
-  // With static weights the weight stream (and its dequantisation into tensor memory) may
-  // start before the previous kernel in the stream has finished; activations, outputs and the
-  // workspace always wait for it.
+  // With static weights the weight stream may start before the previous kernel in the stream
+  // has finished; activations, outputs and the workspace always wait for it.
   if (!p.static_weights) grid_dependency_wait();
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    // One thread feeds three rings, polling whichever has a free slot: packed weights (one
-    // unit per slot), the scale chunks of the 4-bit formats (eight groups x 128 rows, fetched
-    // when a unit begins a new chunk) and activations (one K block per slot; only after the
-    // stream-order wait).
+    // ------------------------------------------------------------ TMA producer: weights and scales
+    // One thread, one ring position per unit, nothing polled that is not needed next: a thread
+    // that looked after all three rings paced the block at one unit per ~650 cycles.
     if (elect_one()) {
-      int iw = 0, ix = 0, ic = 0;                    // units with weights / activations issued, chunks issued
-      int sw = 0, sx = 0, sc = 0;                    // ring slots
-      uint32_t pw = 1, px = 1, pc = 1;               // parity to wait for on the empty barriers
-      int w_tile = tile0, w_kb = kbi0, x_kb = kbi0;
-      bool chunk_done = false;                       // the chunk that unit iw begins has been issued
-      bool waited = !p.static_weights;
+      int iw = 0, ic = 0;                            // units and chunks issued
+      int sw = 0, fw = 0, sc = 0;                    // ring slot, full barrier, chunk slot
+      uint32_t pw = 1, pc = 1;                       // parity to wait for on the empty barriers
+      int tile = tile0, kb = kbi0;
       bool ok = true;
-      uint32_t idle = 0;
-      while (iw < n_units || ix < n_units) {
-        bool progress = false;
-        if (iw < n_units) {
-          const bool chunk_start = kGroups && (iw == 0 || (w_kb & 7) == 0);
-          if (chunk_start && !chunk_done && mbar_test_wait(s_empty + 8 * sc, pc)) {
-            mbar_arrive_expect_tx(s_full + 8 * sc, static_cast<uint32_t>(kSBytes));
-            tma_load_3d(s_ring + sc * kSBytes, &tm_s, s_full + 8 * sc, (w_kb >> 3) * 8, w_tile * kBlockN, 0);
-            if (FMT == FMT_W4_ASYM)
-              tma_load_3d(s_ring + sc * kSBytes + kSkChunkBytes, &tm_z, s_full + 8 * sc, (w_kb >> 3) * 8,
-                          w_tile * kBlockN, 0);
-            chunk_done = true;
-            ++ic;
-            if (++sc == kSkSStages) {
-              sc = 0;
-              pc ^= 1;
-            }
-            progress = true;
-          }
-          if ((!chunk_start || chunk_done) && mbar_test_wait(w_empty + 8 * sw, pw)) {
-            mbar_arrive_expect_tx(w_full + 8 * sw, static_cast<uint32_t>(kWBytes));
-            tma_load_3d(w_ring + sw * kWBytes, &tm_w, w_full + 8 * sw, 0, w_tile * kBlockN,
-                        (FMT == FMT_W8) ? 2 * w_kb : w_kb);
-            ++iw;
-            chunk_done = false;
-            if (++w_kb == KB) {
-              w_kb = 0;
-              ++w_tile;
-            }
-            if (++sw == S) {
-              sw = 0;
-              pw ^= 1;
-            }
-            progress = true;
+      for (; iw < n_units; ++iw) {
+        if (kGroups && (iw == 0 || kb % kChunkUnits == 0)) {
+          ok = wait_or_abort(s_empty + 8 * sc, pc, abort_p);
+          if (!ok) break;
+          const int kbg = kb * kSub;                 // in groups of 128 K
+          mbar_arrive_expect_tx(s_full + 8 * sc, static_cast<uint32_t>(kSBytes));
+          tma_load_3d(s_ring + sc * kSBytes, &tm_s, s_full + 8 * sc, (kbg >> 3) * 8, tile * kBlockN, 0);
+          if (FMT == FMT_W4_ASYM)
+            tma_load_3d(s_ring + sc * kSBytes + kSkChunkBytes, &tm_z, s_full + 8 * sc, (kbg >> 3) * 8, tile * kBlockN, 0);
+          ++ic;
+          if (++sc == kSkSStages) {
+            sc = 0;
+            pc ^= 1;
           }
         }
-        if (!waited && (iw == n_units || !progress)) {
-          // the weight ring is as far ahead as it can get: now order behind the stream
-          grid_dependency_wait();
-          waited = true;
-          progress = true;
+        ok = wait_or_abort(u_empty + 8 * sw, pw, abort_p);
+        if (!ok) break;
+        mbar_arrive_expect_tx(w_full + 8 * fw, static_cast<uint32_t>(kWBytes));
+        tma_load_3d(w_ring + sw * kWBytes, &tm_w, w_full + 8 * fw, 0, tile * kBlockN,
+                    sk_depth(FMT, NT) * kb);
+        if (++kb == KB) {
+          kb = 0;
+          ++tile;
         }
-        if (waited && ix < n_units && mbar_test_wait(x_empty + 8 * sx, px)) {
-          mbar_arrive_expect_tx(x_full + 8 * sx, static_cast<uint32_t>(x_bytes));
-          tma_load_3d(x_ring + sx * x_bytes, &tm_x, x_full + 8 * sx, 0, 0, 2 * x_kb);
-          ++ix;
-          if (++x_kb == KB) x_kb = 0;
-          if (++sx == p.x_stages) {
-            sx = 0;
-            px ^= 1;
-          }
-          progress = true;
+        if (++sw == S) {
+          sw = 0;
+          pw ^= 1;
         }
-        if (progress) {
-          idle = 0;
-        } else {
-          // nothing to do: step aside so this poll loop does not take issue slots from the
-          // dequantising warps that share the scheduler
-          __nanosleep(32);
-          if (++idle > kMaxPolls || ((idle & 0x3FF) == 0 && *abort_p)) {
-            ok = false;
-            break;
-          }
-        }
+        if (++fw == G * S) fw = 0;
       }
       if (!ok) flag_failure(abort_p, p.status, 1u);
       if (*abort_p) {
         // let the copies already in flight land before the block's shared memory is released
-        for (int j = max(0, iw - S); j < iw; ++j) mbar_wait(w_full + 8 * (j % S), (j / S) & 1);
-        for (int j = max(0, ix - p.x_stages); j < ix; ++j) mbar_wait(x_full + 8 * (j % p.x_stages), (j / p.x_stages) & 1);
+        for (int j = max(0, iw - S); j < iw; ++j) mbar_wait(w_full + 8 * (j % (G * S)), (j / (G * S)) & 1);
         for (int j = max(0, ic - kSkSStages); j < ic; ++j) mbar_wait(s_full + 8 * (j % kSkSStages), (j / kSkSStages) & 1);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    // One thread, and every instruction of it is on the block's critical path (a dependent
-    // scalar sequence issues one instruction every several cycles beside the dequantise warps'
-    // bursts): descriptors and ring positions advance incrementally, a segment is counted down.
+    // ------------------------------------------------------------ TMA producer: activations
     if (elect_one()) {
+      grid_dependency_wait();
+      int ix = 0, sx = 0, fx = 0, kb = kbi0;
+      uint32_t px = 1;
       bool ok = true;
-      int sx = 0, as = 0;
-      uint32_t x_phase = 0, a_phase = 0, acc_phase = 1;   // acc_phase: parity to wait for on acc_empty
-      int seg_left = min(KB - kbi0, n_units);             // units left in the current segment (tile)
-      int after_seg = n_units - seg_left;                 // units after it
-      bool seg_first = true;
-      const uint64_t x_desc0 = umma_desc_sw128(x_ring);
-      const uint64_t x_step = static_cast<uint64_t>(x_bytes >> 4), atom_step = static_cast<uint64_t>(x_atom_bytes >> 4);
-      uint64_t x_desc = x_desc0;
-      const uint32_t a_tmem0 = tmem_base + kSkACol0;
-      uint32_t a_tmem = a_tmem0;
-      for (int i = 0; i < n_units; ++i) {
-        if (seg_first) {
-          // the epilogue has read the previous segment out of the accumulator
-          ok = wait_or_abort(acc_empty, acc_phase, abort_p);
-          if (!ok) break;
-          acc_phase ^= 1u;
-        }
-        ok = wait_or_abort(x_full + 8 * sx, x_phase, abort_p) && wait_or_abort(a_full + 8 * as, a_phase, abort_p);
+      for (; ix < n_units; ++ix) {
+        ok = wait_or_abort(u_empty + 8 * sx, px, abort_p);
         if (!ok) break;
-        tc_fence_after_sync();
-        // operand stage `as` holds 128 K elements as 64 columns, 8 per MMA; two 64-K atoms of activations
-        umma_f16_ts(tmem_base, a_tmem, x_desc, p.idesc, seg_first ? 0u : 1u);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) umma_f16_ts(tmem_base, a_tmem + 8 * k, x_desc + 2 * k, p.idesc, 1u);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_f16_ts(tmem_base, a_tmem + 32 + 8 * k, x_desc + atom_step + 2 * k, p.idesc, 1u);
-        umma_commit(a_empty + 8 * as);
-        umma_commit(x_empty + 8 * sx);
-        seg_first = --seg_left == 0;
-        if (seg_first) {
-          umma_commit(acc_full);
-          seg_left = min(KB, after_seg);
-          after_seg -= seg_left;
-        }
-        x_desc += x_step;
-        if (++sx == p.x_stages) {
+        mbar_arrive_expect_tx(x_full + 8 * fx, static_cast<uint32_t>(kXBytes));
+        tma_load_3d(x_ring + sx * kXBytes, &tm_x, x_full + 8 * fx, 0, 0, 2 * kSub * kb);
+        if (++kb == KB) kb = 0;
+        if (++sx == S) {
           sx = 0;
-          x_phase ^= 1;
-          x_desc = x_desc0;
+          px ^= 1;
         }
-        a_tmem += 64;
-        if (++as == kSkAStages) {
-          as = 0;
-          a_phase ^= 1;
-          a_tmem = a_tmem0;
-        }
+        if (++fx == G * S) fx = 0;
       }
       if (!ok) flag_failure(abort_p, p.status, 2u);
+      if (*abort_p)
+        for (int j = max(0, ix - S); j < ix; ++j) mbar_wait(x_full + 8 * (j % (G * S)), (j / (G * S)) & 1);
     }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------ epilogue warps
-    grid_dependency_wait();              // outputs and the workspace belong to the stream order
-    const int quarter = warp & 3;        // TMEM lanes this warp may read
-    const int ch = quarter * 32 + lane;  // channel inside the tile
-    const uint32_t acc_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const int rows = min(p.tok, p.M);
+  } else {
+    // ------------------------------------------------------------ consumer groups
+    // MMA row r of the warp's 16-row tiles is a channel of our choice: lane (gq, t) of the MMA
+    // layout holds rows gq and gq + 8 of each, and gets the 2 MT neighbouring channels from
+    // 2 MT gq on, so that outputs, partials and gated pairs are whole vectors of one lane.  Row i of
+    // the lane is channel 2 MT gq + (i ^ par), par = gq & 1: the eight lanes of a 16-byte
+    // shared-memory phase then touch rows of both parities, i.e. all banks.
+    constexpr bool kGroupSums = Shape::kGroupSums;
+    constexpr int kSlab = Shape::kSlab, kChains = Shape::kChains, kGroupTiles = Shape::kGroupTiles;
+    grid_dependency_wait();                                // activations, outputs and the workspace
+    const int g = (warp - kSkProducers) / kRowWarps;       // group: units g, g + G, ...
+    const int q = (warp - kSkProducers) % kRowWarps;       // which 16 MT channels of the tile
+    const int gq = lane >> 2, t = lane & 3;
+    const int par = gq & 1;
+    // Shared-memory offsets inside a stage; stages are 1024-byte aligned, so the other rows and pieces of the
+    // lane are XORs of low bits: row i sits at w_off ^ ((i & 1) << 6) ^ (i & 2 ? 144 : 0).
+    const int r0 = q * 16 * MT + gq * kChan + par;
+    const uint32_t w_off = static_cast<uint32_t>(r0 * 64 + ((t ^ ((r0 >> 1) & 3)) << 4));
+    // swizzled 16-byte chunk of the lane's activations, token row gq (token tiles are 8 rows: same swizzle)
+    const uint32_t x_off = static_cast<uint32_t>(
+        gq * 128 + (FMT == FMT_W4_ASYM ? (t >> 1) * kXAtom + (((((t & 1) << 2) | ((t >> 1) << 1)) ^ gq) << 4)
+                                       : (((2 * t) ^ gq) << 4)));
+    const uint32_t s_off = static_cast<uint32_t>(r0 * 16);
+    const int rows = min(kTok, p.M);
     T* const y = static_cast<T*>(p.y);
+
     bool ok = true;
-    int tile = tile0, kb = kbi0, left = n_units;
-    uint32_t acc_phase = 0, xg_phase = 0;
-    // one finished fp32 value of this thread's channel -> the output (all lanes take part)
-    auto emit = [&](int m, int n, float v) {
-      if (p.swiglu) {
-        // neighbouring lanes hold the gate (even row) and the up (odd row) of one output channel
-        const float up = __shfl_xor_sync(0xffffffffu, v, 1);
-        if ((lane & 1) == 0 && n < p.N) y[static_cast<int64_t>(m) * p.ldy + (n >> 1)] = from_float<T>(swiglu_pair(v, up));
-      } else if (n < p.N) {
-        y[static_cast<int64_t>(m) * p.ldy + n] = from_float<T>(v);
-      }
-    };
+    int slot = g, full = g, sc = 0;                        // ring slot, full barrier, chunk slot
+    uint32_t u_phase = 0, c_phase = 0, red_phase = 0;
+    int chunk = -1;                                        // the scale chunk in slot sc (-1: none yet)
+    int tile = tile0, kb0 = kbi0, left = n_units, seg = 0; // segment: units [seg, seg + len)
+    int j = g;
     while (left > 0) {
-      const int len = min(left, KB - kb);
-      const int n = tile * kBlockN + ch;
+      const int len = min(left, KB - kb0);
+      float acc[kChains][MT][NT][4];
+#pragma unroll
+      for (int c = 0; c < kChains; ++c)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[c][mt][nt][e] = 0.0f;
+
+      for (; j < seg + len && ok; j += G) {
+        uint32_t group_scale[kChan], group_zero[kChan];    // a pair of groups with the unit's in it, fp16 each
+        if (kGroups) {
+          // unit j lies in chunk (kbi0 + j) / kChunkUnits - kbi0 / kChunkUnits: a tile's units are a
+          // multiple of that, so chunks never straddle tiles.  Every warp takes every chunk in order
+          // and hands the one before it back.
+          const int want = (kbi0 + j) / kChunkUnits - kbi0 / kChunkUnits;
+          while (chunk < want) {                           // at most two steps: a group moves G units at a time
+            if (chunk >= 0) {
+              __syncwarp();
+              if (lane == 0) mbar_arrive(s_empty + 8 * sc);
+              if (++sc == kSkSStages) {
+                sc = 0;
+                c_phase ^= 1;
+              }
+            }
+            ok = wait_or_abort(s_full + 8 * sc, c_phase, abort_p);
+            if (!ok) break;
+            ++chunk;
+          }
+          if (!ok) break;
+          const int group = (kbi0 + j) % kChunkUnits * kSub;       // the unit's first group inside the chunk
+          const uint32_t s_at = s_ring + sc * kSBytes + s_off + (group >> 1) * 4;
+#pragma unroll
+          for (int i = 0; i < kChan; ++i) {
+            group_scale[i] = ld_shared_u32(s_at ^ ((i & 1) << 4) ^ ((i & 2) << 4));
+            if (FMT == FMT_W4_ASYM) group_zero[i] = ld_shared_u32((s_at ^ ((i & 1) << 4) ^ ((i & 2) << 4)) + kSkChunkBytes);
+          }
+        }
+        ok = wait_or_abort(w_full + 8 * full, u_phase, abort_p) && wait_or_abort(x_full + 8 * full, u_phase, abort_p);
+        if (!ok) break;
+#pragma unroll kUnroll
+        for (int sub = 0; sub < kSub; ++sub) {
+        const uint32_t w_at = w_ring + slot * kWBytes + sub * PackedStage<FMT>::kBytes + w_off;
+        const uint32_t x_at = x_ring + slot * kXBytes + sub * 2 * kXAtom + x_off;
+        const int which = kSub == 2 ? sub : (kbi0 + j) & 1;
+        float scale[kChan], zp[kChan];
+        unsigned short scale16[kChan];
+#pragma unroll
+        for (int i = 0; i < kChan; ++i) {
+          scale16[i] = kGroups ? half_bits(group_scale[i], which) : 0;
+          scale[i] = kGroupSums ? __half2float(__ushort_as_half(scale16[i])) : 1.0f;
+          zp[i] = FMT == FMT_W4_ASYM ? __half2float(__ushort_as_half(half_bits(group_zero[i], which))) : 8.0f;
+        }
+        const SkGroup<T, kChan> group_consts(zp, scale16);
+        uint4 packed[kChan];
+#pragma unroll
+        for (int i = 0; i < kChan; ++i) packed[i] = ld_shared_v4(w_at ^ ((i & 1) << 6) ^ ((i & 2) ? 144 : 0));
+        if (FMT == FMT_W4_ASYM && t >= 2) {
+#pragma unroll
+          for (int i = 0; i < kChan; ++i) packed[i] = make_uint4(packed[i].z, packed[i].w, packed[i].x, packed[i].y);
+        }
+        float group_sum[kChains][MT][kGroupTiles][4];      // with kGroupSums: unscaled sums
+        auto slab = [&](auto first_piece) {
+          constexpr int kFirst = decltype(first_piece)::value;
+          if (FMT == FMT_W8 && kFirst == 2) {
+#pragma unroll
+            for (int i = 0; i < kChan; ++i)
+              packed[i] = ld_shared_v4((w_at ^ ((i & 1) << 6) ^ ((i & 2) ? 144 : 0)) + kBlockN * 64);
+          }
+          uint32_t a[kSlab][MT][2][4];
+          Shape::template unpack<kFirst>(packed, group_consts, a[0]);
+          if constexpr (kSlab > 1) Shape::template unpack<kFirst + 1>(packed, group_consts, a[1]);
+          if constexpr (kSlab > 2) {
+            Shape::template unpack<kFirst + 2>(packed, group_consts, a[2]);
+            Shape::template unpack<kFirst + 3>(packed, group_consts, a[3]);
+          }
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            uint4 x[kSlab];
+#pragma unroll
+            for (int s = 0; s < kSlab; ++s)
+              x[s] = ld_shared_v4((x_at ^ piece_flip<FMT>(kFirst + s)) + piece_atom<FMT>(kFirst + s) * kXAtom + nt * 1024);
+#pragma unroll
+            for (int s = 0; s < kSlab; ++s)
+#pragma unroll
+              for (int step = 0; step < 2; ++step)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                  const int c = kChains == 2 ? step : 0;
+                  const uint32_t b0 = step ? x[s].z : x[s].x, b1 = step ? x[s].w : x[s].y;
+                  if constexpr (kGroupSums) {
+                    float(&d)[4] = group_sum[c][mt][Shape::kLocal ? 0 : nt];
+                    if ((Shape::kLocal ? s : kFirst + s) == 0 && (kChains == 2 || step == 0))
+                      mma_16816<T>(d, a[s][mt][step], b0, b1, 0.0f, 0.0f, 0.0f, 0.0f);
+                    else
+                      mma_16816<T>(d, a[s][mt][step], b0, b1, d[0], d[1], d[2], d[3]);
+                  } else {
+                    float(&d)[4] = acc[c][mt][nt];
+                    mma_16816<T>(d, a[s][mt][step], b0, b1, d[0], d[1], d[2], d[3]);
+                  }
+                }
+            if constexpr (kGroupSums) {
+              if (Shape::kLocal || kFirst + kSlab == 4) {
+#pragma unroll
+                for (int c = 0; c < kChains; ++c)
+#pragma unroll
+                  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                      acc[c][mt][nt][e] = fmaf(group_sum[c][mt][Shape::kLocal ? 0 : nt][e], scale[2 * mt + (e >> 1)],
+                                               acc[c][mt][nt][e]);
+              }
+            }
+          }
+        };
+        slab(std::integral_constant<int, 0>{});
+        if constexpr (kSlab == 2) slab(std::integral_constant<int, 2>{});
+        if constexpr (kSlab == 1) {
+          slab(std::integral_constant<int, 1>{});
+          slab(std::integral_constant<int, 2>{});
+          slab(std::integral_constant<int, 3>{});
+        }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(u_empty + 8 * slot);
+        slot += G;
+        if (slot >= S) slot -= S;
+        full += G;
+        if (full >= G * S) {
+          full -= G * S;
+          u_phase ^= 1;
+        }
+      }
+      if (!ok) flag_failure(abort_p, p.status, 4u);
+
+      // ---- end of the segment.  Sums in channel order: sum[nt][h] = the lane's channels of token
+      // 8 nt + 2 t + h.
+      float sum[NT][2][kChan];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < kChan; i += 2) {
+            float v0 = acc[0][i >> 1][nt][h], v1 = acc[0][i >> 1][nt][2 + h];
+            if constexpr (kChains == 2) {
+              v0 += acc[1][i >> 1][nt][h];
+              v1 += acc[1][i >> 1][nt][2 + h];
+            }
+            if (kGroupSums) {
+              v0 *= Nibbles<T>::kInverseUnit;
+              v1 *= Nibbles<T>::kInverseUnit;
+            }
+            sum[nt][h][i] = par ? v1 : v0;
+            sum[nt][h][i + 1] = par ? v0 : v1;
+          }
       // Who else works on this tile: blocks b_lo .. b_hi in unit order.  b_lo (for which the
       // tile is the END of its range, so it finishes it last) owns the tile's output and adds
-      // the others' partials in block order; every other block parks its partial in its own
-      // exchange slot (a block contributes to at most one tile it does not own: the one under
-      // way at the start of its range).
+      // the others' partials; every other block parks its partial in its own exchange slot (a
+      // block contributes to at most one tile it does not own: the one under way at the
+      // start of its range).
       const uint32_t first = static_cast<uint32_t>(tile) * KB;
-      const uint32_t b_lo = (len == KB) ? blockIdx.x : sk_owner(first, G, U);
-      const uint32_t b_hi = (len == KB) ? blockIdx.x : sk_owner(first + KB - 1, G, U);
+      const uint32_t b_lo = (len == KB) ? blockIdx.x : sk_owner(first, grid, U);
+      const uint32_t b_hi = (len == KB) ? blockIdx.x : sk_owner(first + KB - 1, grid, U);
       const bool owner = b_lo == blockIdx.x;
-      float ch_scale = 1.0f, ch_bias = 0.0f;
-      if (owner && n < p.N) {
-        if (FMT == FMT_W8)
-          ch_scale = p.scale_is_f32 ? reinterpret_cast<const float*>(p.scales)[n]
-                                    : __half2float(reinterpret_cast<const __half*>(p.scales)[n]);
-        if (p.bias != nullptr) ch_bias = static_cast<float>(static_cast<const T*>(p.bias)[n]);
-      }
-      const size_t per_slot = static_cast<size_t>(p.tok) * kBlockN;
-      uint32_t* mine = p.exchange + static_cast<size_t>(blockIdx.x) * per_slot + ch;
-      const bool collect = owner && b_hi > b_lo;   // only ever a block's last segment: the rings drain
-      // Up to sixteen token rows: the other blocks' partials are pulled into registers NOW,
-      // while this segment's MMAs are still running (the other blocks finished their part of
-      // the tile earlier), so that nothing but the addition is left once the accumulator is
-      // ready.  Every thread polls its own channel's words (bounded) and empties them.
-      const bool early = collect && rows <= 16;
-      float others[16];
+      const int ch = q * 16 * MT + gq * kChan;             // the lane's first channel in the tile
+      constexpr size_t kSlot = static_cast<size_t>(kTok) * kBlockN;
+      if (owner) {
+        // The groups share the other blocks' partials: group g takes b_lo + 1 + g, b_lo + 1 + g + G, ...
+        // Every lane polls its own words (bounded) and empties them.
+        constexpr int kBatch = NT < 4 ? NT : 4;            // token tiles looked at together
+        for (uint32_t bb = b_lo + 1 + g; bb <= b_hi; bb += G) {
+          uint32_t* const park = p.exchange + bb * kSlot + ch;
 #pragma unroll
-      for (int m = 0; m < 16; ++m) others[m] = 0.0f;
-      if (early) {
-        for (uint32_t bb = b_lo + 1; bb <= b_hi; ++bb) {
-          uint32_t* src = p.exchange + static_cast<size_t>(bb) * per_slot + ch;
-          uint32_t v[16];
-          bool all = false;
-          for (uint32_t tries = 0; !all; ++tries) {
-            all = true;
+          for (int n0 = 0; n0 < NT; n0 += kBatch) {
+            uint32_t v[kBatch][2][kChan];
+            bool all = false;
+            for (uint32_t tries = 0; !all; ++tries) {
+              all = true;
 #pragma unroll
-            for (int m = 0; m < 16; ++m) {
-              v[m] = (m < rows) ? ld_relaxed_gpu_u32(src + m * kBlockN) : 0x80000000u;
-              all = all && v[m] != 0u;
-            }
-            if (!all) {
-              if (tries >= kSkExchangePolls || *abort_p) {
-                atomicOr(p.status, 16u);
-                break;
+              for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  const int m = (n0 + b) * 8 + 2 * t + h;
+#pragma unroll
+                  for (int e = 0; e < kChan; ++e) v[b][h][e] = 0x80000000u;
+                  if (n0 + b < NT && m < rows) ld_exchange(v[b][h], park + m * kBlockN);
+                }
+#pragma unroll
+              for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                  for (int e = 0; e < kChan; ++e) all = all && v[b][h][e] != 0u;
+              if (!all) {
+                if (tries >= kSkExchangePolls || *abort_p) {
+                  atomicOr(p.status, 16u);
+                  break;
+                }
+                __nanosleep(100);
               }
-              __nanosleep(300);
             }
-          }
 #pragma unroll
-          for (int m = 0; m < 16; ++m) {
-            others[m] += sk_decode(v[m]);                            // block order; absent rows add +0.0f
-            if (m < rows) __stcg(src + m * kBlockN, 0u);             // empty again for the next launch
+            for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int m = (n0 + b) * 8 + 2 * t + h;
+                if (n0 + b < NT && m < rows) {
+#pragma unroll
+                  for (int e = 0; e < kChan; ++e) {
+                    sum[n0 + b < NT ? n0 + b : 0][h][e] += sk_decode(v[b][h][e]);
+                    v[b][h][e] = 0u;
+                  }
+                  st_exchange(park + m * kBlockN, v[b][h]);                // empty again for the next launch
+                }
+              }
           }
         }
       }
-      if (ok) {
-        ok = wait_or_abort(acc_full, acc_phase, abort_p);
-        if (!ok) flag_failure(abort_p, p.status, 8u);
-      }
-      acc_phase ^= 1u;
-      tc_fence_after_sync();
-      // Read the accumulator out eight columns (token rows) at a time and hand it back to the
-      // MMA warp as soon as the last of it is in registers.  A tile of this block alone goes
-      // to the output; a partial is parked in this block's exchange slot; an owner's own part
-      // goes to shared memory (the idle activation ring) to have the others' added to it.
-      const uint32_t sum_buf = x_ring + ch * 4;                    // [token row][128 channels] fp32
-      for (int c = 0; c < p.tok; c += 8) {
-        uint32_t r[8];
+      // The other groups hand their sums to group 0 through shared memory: [2 NT][32 lanes] of kChan floats
+      // per warp and group, added in group order.
+      constexpr uint32_t kRedLane = kChan * 4, kRedRow = 32 * kRedLane, kRedWarp = 2 * NT * kRedRow;
+      const uint32_t red_at = red + static_cast<uint32_t>(q) * kRedWarp + static_cast<uint32_t>(lane) * kRedLane;
+      if (g != 0) {
+        ok = ok && wait_or_abort(red_empty + 8 * q, red_phase ^ 1u, abort_p);   // group 0 has read the previous sums
 #pragma unroll
-        for (int j = 0; j < 8; ++j) r[j] = 0u;
-        if (ok) {
-          tmem_ld_x8(acc_addr + c, r);
-          tmem_ld_wait();
-        }
-        if (c + 8 >= p.tok) {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(acc_empty);
-        }
-        if (c >= rows) continue;
-        if (collect && !early) {
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (c + j < rows) st_shared_f32(sum_buf + (c + j) * 512, __uint_as_float(r[j]));
-        } else if (owner) {
-          // (c is 0 or 8 whenever `others` holds anything; otherwise it is all zeros)
+          for (int h = 0; h < 2; ++h)
+            st_shared_f(red_at + (g - 1) * kTok * 512 + (nt * 2 + h) * kRedRow, sum[nt][h]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(red_full + 8 * q);
+      } else {
+        ok = ok && wait_or_abort(red_full + 8 * q, red_phase, abort_p);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float extra = c == 0 ? others[j] : (c == 8 ? others[8 + j] : 0.0f);
-            if (c + j < rows) emit(c + j, n, (__uint_as_float(r[j]) + extra) * ch_scale + ch_bias);
-          }
+        for (int o = 0; o < G - 1; ++o)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              float v[kChan];
+              ld_shared_f(v, red_at + o * kTok * 512 + (nt * 2 + h) * kRedRow);
+#pragma unroll
+              for (int e = 0; e < kChan; ++e) sum[nt][h][e] += v[e];
+            }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(red_empty + 8 * q);
+        if (!owner) {
+          uint32_t* const park = p.exchange + blockIdx.x * kSlot + ch;
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int m = nt * 8 + 2 * t + h;
+              uint32_t v[kChan];
+#pragma unroll
+              for (int e = 0; e < kChan; ++e) v[e] = sk_encode(sum[nt][h][e]);
+              if (m < rows) st_exchange(park + m * kBlockN, v);
+            }
         } else {
+          const int n = tile * kBlockN + ch;
+          float cscale[kChan], cbias[kChan];
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (c + j < rows) __stcg(mine + (c + j) * kBlockN, sk_encode(__uint_as_float(r[j])));
-        }
-      }
-      if (collect && !early) {
-        // More than sixteen token rows.  The other blocks' partials, a batch at a time: one bulk copy per block brings its
-        // whole slot into the idle weight ring (every byte in flight at once: a look costs one
-        // trip to L2 whatever the row count), every thread checks its channel's words, and
-        // the look is repeated (bounded) until none reads as "not written".  Then they are
-        // added in block order and the slots are put back to zero.
-        const uint32_t slot_bytes = static_cast<uint32_t>(rows) * 512u;
-        const uint32_t stride = static_cast<uint32_t>(p.tok) * 512u;
-        const uint32_t room = static_cast<uint32_t>(S) * kWBytes / stride;
-        const uint32_t batch = room < 4u ? (room < 1u ? 1u : room) : 4u;
-        for (uint32_t bb = b_lo + 1; bb <= b_hi; bb += batch) {
-          const uint32_t nb = min(batch, b_hi - bb + 1);
-          bool all = false;
-          for (uint32_t tries = 0; !all; ++tries) {
-            if (threadIdx.x == 64) {
-              mbar_arrive_expect_tx(xg_full, nb * slot_bytes);
-              for (uint32_t z = 0; z < nb; ++z)
-                bulk_load(w_ring + z * stride, p.exchange + static_cast<size_t>(bb + z) * per_slot, slot_bytes, xg_full);
-            }
-            bool landed = wait_or_abort(xg_full, xg_phase, abort_p);
-            xg_phase ^= 1u;
-            bool mine_ok = landed;
-            for (uint32_t z = 0; z < nb && mine_ok; ++z)
-              for (int m = 0; m < rows; ++m)
-                mine_ok = mine_ok && __float_as_uint(ld_shared_f32(w_ring + z * stride + m * 512 + ch * 4)) != 0u;
-            all = epilogue_all(mine_ok);
-            if (!all) {
-              if (tries >= kSkExchangePolls || !landed || *abort_p) {
-                if (threadIdx.x == 64) atomicOr(p.status, 16u);
-                break;
-              }
-              __nanosleep(500);
+          for (int e = 0; e < kChan; ++e) {
+            cscale[e] = 1.0f;
+            cbias[e] = 0.0f;
+            if (n + e < p.N) {
+              if (FMT == FMT_W8)
+                cscale[e] = p.scale_is_f32 ? reinterpret_cast<const float*>(p.scales)[n + e]
+                                           : __half2float(reinterpret_cast<const __half*>(p.scales)[n + e]);
+              if (p.bias != nullptr) cbias[e] = static_cast<float>(static_cast<const T*>(p.bias)[n + e]);
             }
           }
-          for (uint32_t z = 0; z < nb; ++z) {
-            uint32_t* slot = p.exchange + static_cast<size_t>(bb + z) * per_slot + ch;
-            for (int m0 = 0; m0 < rows; m0 += 8) {
-              float a[8], b[8];
+          const bool whole = p.vec_out && n + kChan <= p.N;
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const bool in = m0 + j < rows;
-                a[j] = in ? ld_shared_f32(sum_buf + (m0 + j) * 512) : 0.0f;
-                b[j] = in ? sk_decode(__float_as_uint(ld_shared_f32(w_ring + z * stride + (m0 + j) * 512 + ch * 4))) : 0.0f;
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int m = nt * 8 + 2 * t + h;
+              float v[kChan];
+#pragma unroll
+              for (int e = 0; e < kChan; ++e) v[e] = sum[nt][h][e] * cscale[e] + cbias[e];
+              if (p.argmax) {
+                LaneValues<T, kChan> values;
+#pragma unroll
+                for (int e = 0; e < kChan; ++e) values.v[e] = v[e];
+                argmax_token<T, kChan>(values, n, p.N, m < rows, bars + kSkBestOffset + 8 * m);
+                continue;
               }
+              if (m >= rows) continue;
+              if (p.swiglu) {
+                // neighbouring channels are (gate, up) pairs: MT neighbouring output columns
+                unsigned short* const dst =
+                    reinterpret_cast<unsigned short*>(y + static_cast<int64_t>(m) * p.ldy + (n >> 1));
+                uint32_t two = 0;
+                if constexpr (MT == 2) two = pack_pair<T>(swiglu_pair(v[0], v[1]), swiglu_pair(v[2], v[3]));
+                else two = pack_pair<T>(swiglu_pair(v[0], v[1]), 0.0f);
+                if (MT == 2 && whole) {
+                  *reinterpret_cast<uint32_t*>(dst) = two;
+                } else {
+                  if (n + 1 < p.N) dst[0] = static_cast<unsigned short>(two & 0xFFFFu);
+                  if (MT == 2 && n + 3 < p.N) dst[1] = static_cast<unsigned short>(two >> 16);
+                }
+              } else {
+                unsigned short* const dst = reinterpret_cast<unsigned short*>(y + static_cast<int64_t>(m) * p.ldy + n);
+                uint32_t two[MT];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                if (m0 + j < rows) {
-                  st_shared_f32(sum_buf + (m0 + j) * 512, a[j] + b[j]);
-                  __stcg(slot + (m0 + j) * kBlockN, 0u);             // empty again for the next launch
+                for (int mt = 0; mt < MT; ++mt) two[mt] = pack_pair<T>(v[2 * mt], v[2 * mt + 1]);
+                if (whole) {
+                  if constexpr (MT == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(two[0], two[1]);
+                  else *reinterpret_cast<uint32_t*>(dst) = two[0];
+                } else {
+#pragma unroll
+                  for (int e = 0; e < kChan; ++e)
+                    if (n + e < p.N) dst[e] = static_cast<unsigned short>((e & 1) ? two[e >> 1] >> 16 : two[e >> 1] & 0xFFFFu);
                 }
               }
             }
-          }
-          // every thread is done with the staged batch before the next one overwrites it
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
-        for (int m0 = 0; m0 < rows; m0 += 8) {
-          float v[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = (m0 + j < rows) ? ld_shared_f32(sum_buf + (m0 + j) * 512) : 0.0f;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (m0 + j < rows) emit(m0 + j, n, v[j] * ch_scale + ch_bias);
         }
       }
+      red_phase ^= 1u;
+      seg += len;
       left -= len;
-      kb = 0;
+      kb0 = 0;
       ++tile;
     }
-  } else {
-    // ------------------------------------------------------------ dequantise groups
-    // A warp visits only the units of its group (ring positions advance by the group count: the
-    // bookkeeping of a skipped unit cost as much issue time as it saved); every warp still
-    // takes every scale chunk in order (its row's eight scales into registers), so a chunk slot
-    // is released by exactly eight arrivals.  Unit j lies in chunk ((kbi0 + j) >> 3) - (kbi0 >> 3):
-    // a tile's K blocks are a multiple of eight, so chunks never straddle tiles.
-    const int g = (warp - 6) >> 2;                          // group: units g, g + 2, ...
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;                    // channel inside the tile = TMEM lane
-    const uint32_t row_taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kSkACol0;
-    const int xr = (row >> 1) & 3;                          // 64-byte swizzle term of this row
-    uint4 cs = make_uint4(0u, 0u, 0u, 0u), cz = make_uint4(0u, 0u, 0u, 0u);   // the current chunk
-    bool ok = true;
-    // positions of this group's first unit (the rings are at least two deep, the operand stages three)
-    int kb = kbi0 + g, sw = g, as = g, sc = 0;
-    while (kb >= KB) kb -= KB;
-    uint32_t w_phase = 0, ae_phase = 1, c_phase = 0;
-    int chunks_taken = 0;                                   // scale chunks this warp has consumed
-    for (int j = g; j < n_units && ok; j += kSkGroups) {
-      if (kGroups) {
-        const int chunk = ((kbi0 + j) >> 3) - (kbi0 >> 3);
-        while (chunks_taken <= chunk) {                     // at most two steps: a group moves two units at a time
-          ok = wait_or_abort(s_full + 8 * sc, c_phase, abort_p);
-          if (!ok) break;
-          cs = ld_shared_v4(s_ring + sc * kSBytes + row * 16);
-          if (FMT == FMT_W4_ASYM) cz = ld_shared_v4(s_ring + sc * kSBytes + kSkChunkBytes + row * 16);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(s_empty + 8 * sc);
-          if (++sc == kSkSStages) {
-            sc = 0;
-            c_phase ^= 1;
-          }
-          ++chunks_taken;
+    if (!ok) flag_failure(abort_p, p.status, 4u);
+    if (p.argmax && g == 0) {
+      // This block's keys -> the grid's; the last block of the grid to get here turns those into channel
+      // indices and puts keys and counter back to zero for the next launch.
+      constexpr int kThreads0 = 32 * kRowWarps;
+      const unsigned long long* const best = reinterpret_cast<const unsigned long long*>(generic_base + kSkBestOffset);
+      const int td = threadIdx.x - 32 * kSkProducers;
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads0) : "memory");
+      if (td < rows && td < kSkMaxArgmaxRows && best[td] != 0ull) atomicMax(p.row_keys + td, best[td]);
+      __threadfence();
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads0) : "memory");
+      if (td == 0) abort_p[1] = atomicAdd(p.counter, 1u) == grid - 1u ? 1 : 0;
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads0) : "memory");
+      if (abort_p[1]) {                                    // the last block of the grid
+        __threadfence();
+        if (td < rows && td < kSkMaxArgmaxRows) {
+          const unsigned long long key = __ldcg(p.row_keys + td);
+          static_cast<long long*>(p.y)[td] = static_cast<long long>(0xFFFFFFFFull - (key & 0xFFFFFFFFull)) * (key != 0ull);
+          p.row_keys[td] = 0ull;
         }
-        if (!ok) break;
-      }
-      {
-        PairConsts gp{0u, 0u, 0u};
-        if (kGroups)
-          gp = make_pair_consts(pick_half(cs, kb & 7),
-                                (FMT == FMT_W4_ASYM) ? __half2float(pick_half(cz, kb & 7)) : 8.0f);
-        ok = wait_or_abort(w_full + 8 * sw, w_phase, abort_p);
-        if (!ok) break;
-        const uint32_t w_stage = w_ring + sw * kWBytes;
-        const uint32_t a_stage_t = row_taddr + as * 64;
-        if (FMT == FMT_W4_REF) {
-          // 64 bytes of the row: byte j holds K j (low nibble) and K 64 + j (high nibble)
-          const uint32_t prow = w_stage + row * 64;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t lo[16], hi[16];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const uint4 v = ld_shared_v4(prow + (((2 * h + c) ^ xr) << 4));
-              const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int w = 0; w < 4; ++w) {
-                // bytes (b0,b1,b2,b3) -> (b0,b2,b1,b3): the masks then pick (b0,b1) from the
-                // word and (b2,b3) from the word shifted by 8
-                const uint32_t u = prmt(words[w], 0u, 0x3120);
-                lo[(c * 4 + w) * 2] = deq_lo<T>(u, gp);
-                lo[(c * 4 + w) * 2 + 1] = deq_lo<T>(u >> 8, gp);
-                hi[(c * 4 + w) * 2] = deq_hi<T>(u, gp);
-                hi[(c * 4 + w) * 2 + 1] = deq_hi<T>(u >> 8, gp);
-              }
-            }
-            if (h == 0) {
-              ok = wait_or_abort(a_empty + 8 * as, ae_phase, abort_p);
-              if (!ok) break;
-              tc_fence_after_sync();
-            }
-            tmem_st_x16(a_stage_t + 16 * h, lo);
-            tmem_st_x16(a_stage_t + 32 + 16 * h, hi);
-          }
-        } else if (FMT == FMT_W4_ASYM) {
-          // 16 words of the row, word w = K 8w .. 8w+7; the layout's nibble order makes every
-          // lop3 pair a pair of K neighbours
-          const uint32_t prow = w_stage + row * 64;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 v = ld_shared_v4(prow + ((c ^ xr) << 4));
-            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-            uint32_t out[16];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              const uint32_t u = words[w];
-              out[w * 4 + 0] = deq_lo<T>(u, gp);        // inputs 0,1
-              out[w * 4 + 1] = deq_hi<T>(u, gp);        // inputs 2,3
-              out[w * 4 + 2] = deq_lo<T>(u >> 8, gp);   // inputs 4,5
-              out[w * 4 + 3] = deq_hi<T>(u >> 8, gp);   // inputs 6,7
-            }
-            if (c == 0) {
-              ok = wait_or_abort(a_empty + 8 * as, ae_phase, abort_p);
-              if (!ok) break;
-              tc_fence_after_sync();
-            }
-            tmem_st_x16(a_stage_t + 16 * c, out);
-          }
-        } else {
-          // int8: two [128 x 64 B] sub-tiles (K 0..63, 64..127).  The integers enter the MMA
-          // unscaled (exact in fp16 and bf16); the channel scale is applied to the accumulator.
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const uint32_t sub = w_stage + (h >> 1) * (kBlockN * 64) + row * 64;
-            uint32_t out[16];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const uint4 v = ld_shared_v4(sub + (((2 * (h & 1) + c) ^ xr) << 4));
-              const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int w = 0; w < 4; ++w) {
-                __half2 k01, k23;
-                int8x4_to_h2(words[w], k01, k23);
-                out[(c * 4 + w) * 2] = pack_operand<T>(k01);
-                out[(c * 4 + w) * 2 + 1] = pack_operand<T>(k23);
-              }
-            }
-            if (h == 0) {
-              ok = wait_or_abort(a_empty + 8 * as, ae_phase, abort_p);
-              if (!ok) break;
-              tc_fence_after_sync();
-            }
-            tmem_st_x16(a_stage_t + 16 * h, out);
-          }
-        }
-        if (!ok) break;
-        tmem_st_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(a_full + 8 * as);
-          mbar_arrive(w_empty + 8 * sw);
-        }
-      }
-      kb += kSkGroups;
-      while (kb >= KB) kb -= KB;                          // (a one-block K wraps twice)
-      sw += kSkGroups;
-      if (sw >= S) {
-        sw -= S;
-        w_phase ^= 1;
-      }
-      as += kSkGroups;
-      if (as >= kSkAStages) {
-        as -= kSkAStages;
-        ae_phase ^= 1;
+        if (td == 0) *p.counter = 0u;
       }
     }
-    if (!ok) flag_failure(abort_p, p.status, 4u);
-  }
-
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem_base, kSkTmemCols);
   }
 }
 
 // ---------------------------------------------------------------- host side
 struct SkPlan {
-  int tok, n_tiles, kb_total, stages, x_stages, grid;
+  int nt;                // token tiles of eight rows the kernel is instantiated for
+  int tok, n_tiles, kb_total, stages, grid;
   uint32_t units;
   size_t smem_bytes;
 };
@@ -751,25 +931,29 @@ static bool sk_geometry(int format, int M, int N, int K) {
 
 static SkPlan sk_plan(int format, int M, int N, int K, int sms) {
   SkPlan pl{};
-  pl.tok = (M + 15) / 16 * 16;
+  pl.nt = M <= 8 ? 1 : (M <= 16 ? 2 : (M <= 32 ? 4 : (M <= 48 ? 6 : 8)));
+  pl.tok = 8 * pl.nt;
   pl.n_tiles = (N + kBlockN - 1) / kBlockN;
-  pl.kb_total = K / kBlockK;
+  pl.kb_total = K / kBlockK / sk_sub(format, pl.nt);
   pl.units = static_cast<uint32_t>(pl.n_tiles) * static_cast<uint32_t>(pl.kb_total);
-  // at least four units per block: a block's set-up must be worth its share
-  const uint32_t want = pl.units / 4;
-  pl.grid = static_cast<int>(std::max<uint32_t>(1u, std::min<uint32_t>(static_cast<uint32_t>(std::min(sms, kSkMaxGrid)), want)));
-  // Shared memory: half an SM when that leaves the weight ring at least six stages (so that
-  // the next kernel's block fits beside this one), otherwise the whole SM.
-  const size_t w_stage = format == FMT_W8 ? kBlockN * 128 : kBlockN * 64;
+  // at least 32 KB of weights per block: its set-up must be worth its share
+  const uint32_t want = pl.units * static_cast<uint32_t>(sk_depth(format, pl.nt)) / 4;
+  // One block per SM, which leaves room for the next kernel's; two for an output head, four tiles or more per SM, where
+  // twice the warps are worth more than the head start of the next kernel: 151936 x 4096, 16 rows, fp16 / bf16
+  // 117 / 110 -> 99 / 91 us.  (24576 x 4096 alone gains as well, 22.5 -> 20.5 us, but a decode step of such matrices
+  // in which different kernels follow one another loses: 166 -> 189 us.)
+  uint32_t blocks = static_cast<uint32_t>(std::min(sms, kSkMaxSms));
+  if (pl.nt <= 2 && pl.units >= 4 * blocks * static_cast<uint32_t>(pl.kb_total)) blocks *= 2;
+  pl.grid = static_cast<int>(std::max<uint32_t>(1u, std::min<uint32_t>(blocks, want)));
+  // Shared memory: half an SM up to 16 token rows (so that the next kernel's block fits beside
+  // this one: at least four stages, i.e. 64 KB of weights in flight), otherwise the whole SM.
+  const size_t stage = static_cast<size_t>(sk_depth(format, pl.nt)) * kBlockN * 64 + static_cast<size_t>(sk_sub(format, pl.nt)) * pl.tok * 256;
   const size_t chunk = format == FMT_W8 ? 0 : static_cast<size_t>(kSkChunkBytes) * (format == FMT_W4_ASYM ? 2 : 1);
-  // wide token tiles keep two activation stages (16 KB each at 64 rows; the collecting owner
-  // needs rows x 512 bytes of the ring as its summing buffer), so that the block still fits half an SM
-  pl.x_stages = pl.tok > 32 ? 2 : kSkXStages;
-  const size_t fixed = 1024 + kSkBarrierBytes + static_cast<size_t>(pl.x_stages) * pl.tok * 256 + kSkSStages * chunk;
-  int stages = kSkHalfSm > fixed ? static_cast<int>((kSkHalfSm - fixed) / w_stage) : 0;
-  if (stages < 6) stages = static_cast<int>((kSkFullSm - fixed) / w_stage);
+  const size_t fixed = 1024 + kSkBarrierBytes + kSkSStages * chunk + static_cast<size_t>(kSkGroups - 1) * pl.tok * 512;
+  int stages = pl.nt <= 2 ? static_cast<int>((kSkHalfSm - fixed) / stage) : 0;
+  if (stages < 4) stages = static_cast<int>((kSkFullSm - fixed) / stage);
   pl.stages = std::max(2, std::min(stages, kSkMaxStages));
-  pl.smem_bytes = fixed + static_cast<size_t>(pl.stages) * w_stage;
+  pl.smem_bytes = fixed + static_cast<size_t>(pl.stages) * stage;
   return pl;
 }
 
@@ -779,7 +963,7 @@ size_t sk_workspace_bytes(int format, int M, int N, int K) {
 }
 
 bool sk_supported(const ForwardArgs& a) {
-  if (a.argmax) return false;
+  if (a.argmax && a.M > kSkMaxArgmaxRows) return false;
   if (a.gather != nullptr && a.gather->world > 1) return false;
   if (a.reduce != nullptr && a.reduce->world > 1) return false;
   if (a.format != FMT_W8) {
@@ -790,15 +974,22 @@ bool sk_supported(const ForwardArgs& a) {
   return sk_geometry(a.format, a.M, a.N, a.K);
 }
 
-// Where the stream-K kernel measured faster than the tile kernel (B200, CUDA-graph replay over
-// rotating weights): 4-bit weights at up to sixteen token rows when a weight tile is shared by
-// few blocks (a block's share of units is at least half a tile's K), e.g. 4096 -> 12288 at
-// M = 1 / 16: 12.3 / 14.2 us against 14.1 / 15.0.  It lost on int8 (4096 -> 12288 M = 16: 18.3
-// against 16.9 us), on deep K (12288 -> 4096 M = 16: 17.2 against 16.0) and above sixteen rows.
+// Where the stream-K kernel measured faster than the tile kernel (B200, bf16, CUDA-graph replay over
+// rotating weights): up to 32 token rows, on weights large enough that streaming them outlasts the
+// hand-over of partial sums between blocks.  us against the tile kernel's, 4-bit:
+//   24576 x 4096 M = 8 / 16 / 32: 15.4 / 20.5 / 26.1 against ~28 / 29 / 33.3;  4096 x 12288 M = 8 / 16 /
+//   32: 10.2 / 13.3 / 17.8 against 16.6 / 17.0 / 20.1;  4096 x 4096 M = 16 / 32 (8 MB): 7.9 / 10.4 against
+//   8.5 / 10.9;  2048 x 2048 M = 8 / 16 (2 MB): 4.9 / 6.7 against 4.6 / 4.9;
+// int8: 24576 x 4096 M = 8 / 16 / 32: 22.0 / 23.6 / 29.2 against 29.7 / 29.7 / 32.3;  4096 x 4096 M = 8 /
+//   32: 7.6 / 11.4 against 9.3 / 12.5;  2048 x 2048 M = 8 / 16 (4 MB): 6.0 / 7.7 against 5.6 / 5.7.
+// Above 32 rows mma.sync bounds it (4-bit 24576 x 4096 M = 40: 38.9 against 34.8).  A weight tile shared by
+// few blocks (a block's share is at least half a tile's K) has little to hand over and pays from 4 MB.
 bool sk_preferred(int format, int M, int N, int K) {
-  if (format == FMT_W8 || M > 16 || !sk_geometry(format, M, N, K)) return false;
+  if (M > 32 || !sk_geometry(format, M, N, K)) return false;
   const SkPlan pl = sk_plan(format, M, N, K, sm_count());
-  return 2u * (pl.units / static_cast<uint32_t>(pl.grid)) >= static_cast<uint32_t>(pl.kb_total);
+  const bool few = 2u * (pl.units / static_cast<uint32_t>(pl.grid)) >= static_cast<uint32_t>(pl.kb_total);
+  const int64_t bytes = static_cast<int64_t>(N) * K / (format == FMT_W8 ? 1 : 2);
+  return bytes >= (few ? (4ll << 20) : (7ll << 20));
 }
 
 int sk_gather_arrivals(int, int, int, int) { return 0; }
@@ -806,14 +997,16 @@ int sk_gather_arrivals(int, int, int, int) { return 0; }
 bool sk_describe(int format, int M, int N, int K, char* text, size_t size) {
   if (!sk_geometry(format, M, N, K)) return false;
   const SkPlan pl = sk_plan(format, M, N, K, sm_count());
-  std::snprintf(text, size, "wq_gemm_sk_kernel<%s> tok=%d units=%u grid=%d ring=%d smem=%zu",
+  std::snprintf(text, size, "wq_gemm_sk_kernel_mma<%s> tok=%d units=%u grid=%d ring=%d smem=%zu",
                 format == FMT_W8 ? "w8" : (format == FMT_W4_REF ? "w4_ref" : "w4_asym"), pl.tok, pl.units,
                 pl.grid, pl.stages, pl.smem_bytes);
   return true;
 }
 
-template <int FMT, typename T>
+template <int FMT, typename T, int NT>
 static int launch_sk_typed(const ForwardArgs& a, const SkPlan& pl) {
+  using Shape = SkShape<FMT, T, NT, kSkTiles, kSkGroups>;
+  const auto kernel = wq_gemm_sk_kernel_mma<FMT, T, NT, kSkTiles, kSkGroups>;
   static bool attr_set_dev[64] = {};
   static std::mutex attr_mu;
   {
@@ -822,13 +1015,13 @@ static int launch_sk_typed(const ForwardArgs& a, const SkPlan& pl) {
     bool& attr_set = attr_set_dev[dev & 63];
     std::lock_guard<std::mutex> g(attr_mu);
     if (!attr_set) {
-      cudaError_t e = cudaFuncSetAttribute(wq_gemm_sk_kernel<FMT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            static_cast<int>(kSkFullSm));
       if (e != cudaSuccess) {
         set_last_error("cudaFuncSetAttribute", e);
         return B200Q_ERR_CUDA;
       }
-      (void)cudaFuncSetAttribute(wq_gemm_sk_kernel<FMT, T>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      (void)cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
       (void)cudaGetLastError();
       attr_set = true;
@@ -839,14 +1032,14 @@ static int launch_sk_typed(const ForwardArgs& a, const SkPlan& pl) {
   // for int4, two such (K 0..63 and 64..127) for int8.  Read one row per thread: 64-byte swizzle.
   const uint64_t w_row_bytes = (FMT == FMT_W8) ? static_cast<uint64_t>(a.K) : static_cast<uint64_t>(a.K / 2);
   if (!get_tensor_map(&tm_w, a.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 64, static_cast<uint64_t>(a.N),
-                      w_row_bytes / 64, static_cast<uint64_t>(a.ldw), 64, 64, kBlockN, (FMT == FMT_W8) ? 2u : 1u,
+                      w_row_bytes / 64, static_cast<uint64_t>(a.ldw), 64, 64, kBlockN, static_cast<uint32_t>(sk_depth(FMT, NT)),
                       CU_TENSOR_MAP_SWIZZLE_64B))
     return B200Q_ERR_CUDA;
   // Activations as {64 elements, M rows, K atoms}: a box of depth 2 is one K block.
   const CUtensorMapDataType xdt = (a.act_dtype == B200Q_F16) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                              : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   if (!get_tensor_map(&tm_x, a.x, xdt, 64, static_cast<uint64_t>(a.M), static_cast<uint64_t>(a.K / 64),
-                      static_cast<uint64_t>(a.ldx) * 2, 128, 64, static_cast<uint32_t>(pl.tok), 2,
+                      static_cast<uint64_t>(a.ldx) * 2, 128, 64, static_cast<uint32_t>(pl.tok), 2u * sk_sub(FMT, NT),
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return B200Q_ERR_CUDA;
   // Scales (and zero-points) as {K / 128 groups, N rows, 1} fp16: a box is eight groups of 128
@@ -873,22 +1066,23 @@ static int launch_sk_typed(const ForwardArgs& a, const SkPlan& pl) {
   p.M = a.M;
   p.N = a.N;
   p.K = a.K;
-  p.tok = pl.tok;
   p.kb_total = pl.kb_total;
   p.total_units = pl.units;
   p.stages = pl.stages;
-  p.x_stages = pl.x_stages;
-  const uint32_t ab_fmt = a.act_dtype == B200Q_F16 ? 0u : 1u;    // both operands in the activation dtype
-  p.idesc = umma_idesc_f16(ab_fmt, ab_fmt, 128u, static_cast<uint32_t>(pl.tok));
+  p.vec_out = (a.swiglu ? a.ldy % 2 == 0 && reinterpret_cast<uintptr_t>(a.y) % 4 == 0
+                        : a.ldy % 4 == 0 && reinterpret_cast<uintptr_t>(a.y) % 8 == 0) ? 1 : 0;
   p.static_weights = a.static_weights ? 1 : 0;
   p.swiglu = a.swiglu ? 1 : 0;
+  p.argmax = a.argmax ? 1 : 0;
   uint8_t* ws = static_cast<uint8_t*>(a.workspace);
   p.status = reinterpret_cast<unsigned*>(ws);
+  p.counter = reinterpret_cast<unsigned*>(ws + kWsCountersOffset);
+  p.row_keys = reinterpret_cast<unsigned long long*>(ws + kWsKeysOffset);
   p.exchange = reinterpret_cast<uint32_t*>(ws + kWsExchangeOffset);
 
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(pl.grid);
-  cfg.blockDim = dim3(kSkThreads);
+  cfg.blockDim = dim3(Shape::kThreads);
   cfg.dynamicSmemBytes = pl.smem_bytes;
   cfg.stream = a.stream;
   cudaLaunchAttribute attr[1];
@@ -901,12 +1095,23 @@ static int launch_sk_typed(const ForwardArgs& a, const SkPlan& pl) {
                  "b200q plan: stream-K kernel fmt %d M %d N %d K %d | tok %d tiles %d kb %d units %u grid %d | "
                  "weight ring %d stages | smem %zu\n",
                  FMT, a.M, a.N, a.K, pl.tok, pl.n_tiles, pl.kb_total, pl.units, pl.grid, pl.stages, pl.smem_bytes);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, wq_gemm_sk_kernel<FMT, T>, tm_w, tm_x, tm_s, tm_z, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_w, tm_x, tm_s, tm_z, p);
   if (e != cudaSuccess) {
     set_last_error("cudaLaunchKernelEx", e);
     return B200Q_ERR_CUDA;
   }
   return note_launch();
+}
+
+template <int FMT, typename T>
+static int launch_sk_width(const ForwardArgs& a, const SkPlan& pl) {
+  switch (pl.nt) {
+    case 1: return launch_sk_typed<FMT, T, 1>(a, pl);
+    case 2: return launch_sk_typed<FMT, T, 2>(a, pl);
+    case 4: return launch_sk_typed<FMT, T, 4>(a, pl);
+    case 6: return launch_sk_typed<FMT, T, 6>(a, pl);
+    default: return launch_sk_typed<FMT, T, 8>(a, pl);
+  }
 }
 
 int launch_forward_sk(const ForwardArgs& a) {
@@ -915,11 +1120,11 @@ int launch_forward_sk(const ForwardArgs& a) {
   const bool h = a.act_dtype == B200Q_F16;
   switch (a.format) {
     case FMT_W8:
-      return h ? launch_sk_typed<FMT_W8, __half>(a, pl) : launch_sk_typed<FMT_W8, __nv_bfloat16>(a, pl);
+      return h ? launch_sk_width<FMT_W8, __half>(a, pl) : launch_sk_width<FMT_W8, __nv_bfloat16>(a, pl);
     case FMT_W4_REF:
-      return h ? launch_sk_typed<FMT_W4_REF, __half>(a, pl) : launch_sk_typed<FMT_W4_REF, __nv_bfloat16>(a, pl);
+      return h ? launch_sk_width<FMT_W4_REF, __half>(a, pl) : launch_sk_width<FMT_W4_REF, __nv_bfloat16>(a, pl);
     case FMT_W4_ASYM:
-      return h ? launch_sk_typed<FMT_W4_ASYM, __half>(a, pl) : launch_sk_typed<FMT_W4_ASYM, __nv_bfloat16>(a, pl);
+      return h ? launch_sk_width<FMT_W4_ASYM, __half>(a, pl) : launch_sk_width<FMT_W4_ASYM, __nv_bfloat16>(a, pl);
     default:
       return B200Q_ERR_INVALID;
   }

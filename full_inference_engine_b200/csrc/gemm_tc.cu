@@ -1570,7 +1570,12 @@ int launch_forward_tc(const ForwardArgs& a) {
   if (a.workspace == nullptr) return B200Q_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(a.workspace) % 256) return B200Q_ERR_ALIGNMENT;
   if (a.force_streamk && !sk_supported(a)) return B200Q_ERR_UNSUPPORTED;
-  if (sk_supported(a) && (a.force_streamk || sk_preferred(a.format, a.M, a.N, a.K))) return launch_forward_sk(a);
+  // The stream-K kernel wants its exchange region.  Calls that it took over from this kernel (int8, more than
+  // sixteen rows, the argmax) keep working on the smaller workspace that this kernel is content with.
+  if (sk_supported(a) && (a.force_streamk || sk_preferred(a.format, a.M, a.N, a.K))) {
+    const bool optional = !a.force_streamk && (a.argmax || a.format == FMT_W8 || a.M > 16);
+    if (!optional || a.workspace_bytes >= kWsExchangeOffset + kWsExchangeBytes) return launch_forward_sk(a);
+  }
   // The fused argmax never splits K: it needs the header (counters and row keys) only.
   if (a.argmax && a.M > kMaxArgmaxRows) return B200Q_ERR_UNSUPPORTED;
   // (nor does the fused all-reduce: a rank's K shard is already a K split)
