@@ -1157,6 +1157,52 @@ static int packed_stage_bytes(int format) { return format == FMT_W8 ? kBlockN * 
 // Most weight tiles a problem may have for its 33..64-token tiles to take the wide block shape.
 constexpr int kWideSmallMaxTiles = 74;
 
+// Clusters of `s` blocks that are resident at once, each block owning its SM (`per_sm` = 1) or half of one: a cluster stays
+// inside a group of 16 to 20 SMs, of which the chip has eight.  (48 clusters of three do not fit: 6144 x 4096 int8,
+// M = 144 / 256, three splits through the workspace 19.5 / 27.8 us, two in a cluster 15.4 / 21.0.)
+static int resident_clusters(int s, int per_sm) { return 8 * (16 * per_sm / s); }
+
+// Problems of one wave (33 to 256 tokens, few weight tiles): token tile, K split and block shape together.  Such a
+// launch is a latency: set-up, a K block after another, the epilogue's rows, a split's reduction.  Its cost in us,
+// fitted to sweeps of 1024..6144 x 1024..4096 at M = 40..256, int8 fp16 and 4-bit bf16 (within 10 % of most):
+//   1.7 + 0.0137 per token row (0.019 above 128) + K blocks x max(unpack, MMA) + 1.9 / 2.5 for two / more splits
+// with 0.42 (int8) or 0.60 (4-bit) to unpack a K block with sixteen warps, more with eight, and 0.0021 per token row to
+// multiply it; 0.9 when blocks that own an SM leave the next kernel of the stream fewer than half of them, 1.0 for
+// int8 blocks of half an SM (their neighbours in a real layer sequence were slower: eight layers of 56 projections at
+// M = 144 362 us without this term, 346 with it; six splits, good in isolation, cost 50 us there and are not tried).
+// One tile of all tokens on as many SMs as there are weight tiles was the rule before: int8 M = 144, 1024 x 1024
+// 7.4 -> 5.3, 3072 x 1024 7.5 -> 5.9, 1024 x 3072 9.9 -> 7.7; M = 256, 2048 x 2048 13.1 -> 8.9.
+struct OneWave {
+  int tok = 0, splits = 1;
+  bool wide = false;
+};
+static OneWave one_wave_plan(int format, int M, int n_tiles, int kb_total, bool no_split) {
+  OneWave best;
+  double best_cost = 0.0;
+  for (int mt = 1; mt <= 8; ++mt) {
+    for (int wide = 1; wide >= 0; --wide) {
+      const int step = wide ? 32 : 16;         // sixteen dequantise warps: four column slices of eight-column groups
+      const int tok = ((M + mt - 1) / mt + step - 1) / step * step;
+      if (!wide && tok > 64) continue;
+      const int tiles = (M + tok - 1) / tok * n_tiles;
+      for (int s = 1; s <= 4; s *= 2) {
+        const int kbs = (kb_total + s - 1) / s;
+        if (s > 1 && (no_split || kbs < 4 || tiles > resident_clusters(s, wide ? 1 : 2))) continue;
+        if (tiles * s > 148) continue;
+        const double unpack = (format == FMT_W8 ? 0.42 : 0.60) * (wide ? 1.0 : (tok > 48 ? 1.45 : 1.15));
+        const double cost = (tok <= 128 ? 1.7 + 0.0137 * tok : 3.45 + 0.019 * (tok - 128)) +
+                            kbs * std::max(unpack, 0.0021 * tok) + (s == 1 ? 0.0 : (s == 2 ? 1.9 : 2.5)) +
+                            (wide && tiles * s > 74 ? 0.9 : 0.0) + (!wide && format == FMT_W8 ? 1.0 : 0.0);
+        if (best.tok == 0 || cost < best_cost - 1e-9) {
+          best_cost = cost;
+          best = OneWave{tok, s, wide != 0};
+        }
+      }
+    }
+  }
+  return best;
+}
+
 static TcPlan make_plan(int format, int M, int N, int K, bool no_split = false) {
   TcPlan pl{};
   // Token tile: as few tiles as cover M, except that a problem of at most two waves (148
@@ -1196,8 +1242,18 @@ static TcPlan make_plan(int format, int M, int N, int K, bool no_split = false) 
   // better with them.  Each of the four column slices must then be whole groups of 8 columns.
   pl.dw = 8;
   const int tiles0 = mt * ((N + kBlockN - 1) / kBlockN);
-  const bool wide = tok > 64 || (tok > 32 && tiles0 <= kWideSmallMaxTiles && (K + kBlockK - 1) / kBlockK >= 32);
-  if (wide && mt < 4) {
+  const int kb_all = (K + kBlockK - 1) / kBlockK;
+  bool wide = tok > 64 || (tok > 32 && tiles0 <= kWideSmallMaxTiles && kb_all >= 32);
+  // (Deeper K keeps the rule below: its splits outnumber a cluster's blocks.  So do 33..64 tokens from 32 K blocks
+  // on, where streaming the weights is most of the time.)
+  OneWave small;
+  if (M > 32 && M <= 256 && kb_all <= 48 && (M > 64 || kb_all < 32) && tiles0 <= 148)
+    small = one_wave_plan(format, M, (N + kBlockN - 1) / kBlockN, kb_all, no_split);
+  if (small.tok > 0) {
+    tok = small.tok;
+    wide = small.wide;
+    if (wide) pl.dw = 16;
+  } else if (wide && mt < 4) {
     tok = (tok + 31) / 32 * 32;
     pl.dw = 16;
   }
@@ -1258,14 +1314,22 @@ static TcPlan make_plan(int format, int M, int N, int K, bool no_split = false) 
   if (max_splits > 16) max_splits = 16;
   if (max_splits < 1) max_splits = 1;
   int best = 1;
-  if (wide) {
+  if (small.tok > 0) {
+    best = small.splits;
+  } else if (wide) {
     if (2 * tiles <= slots) {
       best = slots / tiles;
-      const int cap = pl.kb_total / 8;         // a wide tile's split must be worth its reduction
+      // a wide tile's split must be worth its reduction: eight K blocks, five where few tiles leave most SMs idle
+      // (1024 x 4096 int8 M = 40: four splits 7.8, six 6.7 us)
+      const int cap = pl.kb_total / (tiles <= 16 && pl.kb_total <= 48 ? 5 : 8);
       if (best > cap) best = cap;
       if (best > max_splits) best = max_splits;
+      // reduced inside clusters that are all resident, if fewer splits get there
+      while (best > 2 && best <= 8 && tiles > resident_clusters(best, 1)) --best;
     }
-  } else {
+  } else if (tiles < 148) {
+    // (From 148 tiles on the partials cost more than the half-filled wave: 24576 x 4096 M = 61, three splits / one:
+    // int8 39.6 / 32.8 us, 4-bit 40.3 / 38.2.)
     double best_eff = 0.0;
     for (int s = 1; s <= max_splits; ++s) {
       const int ctas = tiles * s;
