@@ -52,15 +52,14 @@ def _forward(inputs, packed, scales, zeros, bias, group_size, kernel, where, sta
     need = _lib.workspace_bytes(4, m, n, k)
     ws = _lib.workspace_for(inputs.device, need)
     layout = _lib.W4_REF_SPLIT_HALF_SYM if zeros is None else _lib.W4_ASYM_ZP_INT32
-    with torch.cuda.device(inputs.device):
-        _lib.check(_lib.library().b200q_w4a16_forward(
-            x.data_ptr(), x.stride(0), _lib.dtype_enum(x.dtype),
-            w.data_ptr(), w.stride(0) * w.element_size(), layout,
-            s.data_ptr(), None if z is None else z.data_ptr(), group_size,
-            None if b is None else b.data_ptr(),
-            out.data_ptr(), out.stride(0), m, n, k,
-            ws.data_ptr(), ws.numel(), kernel | flags,
-            _lib.stream_ptr(inputs.device)), where)
+    _lib.check(_lib.call_on(
+        inputs.device, _lib.library().b200q_w4a16_forward,
+        x.data_ptr(), x.stride(0), _lib.dtype_enum(x.dtype),
+        w.data_ptr(), w.stride(0) * w.element_size(), layout,
+        s.data_ptr(), None if z is None else z.data_ptr(), group_size,
+        None if b is None else b.data_ptr(),
+        out.data_ptr(), out.stride(0), m, n, k,
+        ws.data_ptr(), ws.numel(), kernel | flags), where)
     return out
 
 

@@ -88,14 +88,11 @@ def w8a16_linear(inputs: torch.Tensor, qweight: torch.Tensor, scales: torch.Tens
     flags = (_lib.FLAG_STATIC_WEIGHTS if static_weights else 0) \
         | (_lib.FLAG_SWIGLU_PAIRS if swiglu_pairs else 0) | (_lib.FLAG_ARGMAX if _argmax else 0)
     ws = _lib.workspace_for(inputs.device, _lib.workspace_bytes(8, m, n, k))
-    with torch.cuda.device(inputs.device):
-        _lib.check(_lib.library().b200q_w8a16_forward(
-            x.data_ptr(), x.stride(0), _lib.dtype_enum(x.dtype),
-            w.data_ptr(), w.stride(0), s.data_ptr(), _lib.dtype_enum(s.dtype),
-            None if b is None else b.data_ptr(),
-            out.data_ptr(), out.stride(0), m, n, k,
-            ws.data_ptr(), ws.numel(),
-            _KERNELS[kernel] | flags,
-            _lib.stream_ptr(inputs.device)),
-            "w8a16_linear")
+    _lib.check(_lib.call_on(
+        inputs.device, _lib.library().b200q_w8a16_forward,
+        x.data_ptr(), x.stride(0), _lib.dtype_enum(x.dtype),
+        w.data_ptr(), w.stride(0), s.data_ptr(), _lib.dtype_enum(s.dtype),
+        None if b is None else b.data_ptr(),
+        out.data_ptr(), out.stride(0), m, n, k,
+        ws.data_ptr(), ws.numel(), _KERNELS[kernel] | flags), "w8a16_linear")
     return out
