@@ -1,5 +1,5 @@
-// Pieces shared by the two tcgen05 kernels (gemm_tc.cu: one block per output tile, every
-// M; gemm_sk.cu: persistent stream-K blocks for decode-sized M): tile constants, bounded
+// Pieces shared by the two tensor-core kernels (gemm_tc.cu: tcgen05, one block per output tile, every
+// M; gemm_sk.cu: mma.sync, persistent stream-K blocks for decode-sized M): tile constants, bounded
 // waits, register-level dequantisation into the fp16 MMA operand, epilogue conversions,
 // the workspace layout and the host-side tensor-map cache.
 //
